@@ -241,54 +241,8 @@ __global__ void scale_rows_kernel(const float2 *in, long long in_rs, float2 *out
 }
 
 // ---------------------------------------------------------------------------
-// Kernel table: [logn][mode][variant], variant 0 = 256-thread CTAs, 1 = 512.
-template <int LOGN, int MODE, int T, int EPTW = 32>
-static KernelInfo make_info()
-{
-  using S = Sched<LOGN, T, EPTW>;
-  KernelInfo k;
-  k.fn = (const void *)&rows_kernel<LOGN, MODE, T, EPTW>;
-  k.ept = EPTW;
-  k.threads = T;
-  k.cluster = S::CS;
-  k.rows_per_cta = S::ROWS;
-  k.smem = S::SMEM;
-  k.tw_bytes = S::tw_bytes();
-  return k;
-}
-
-
-template <int LOGN>
-static void fill_table(KernelInfo (*tab)[3][kVariants])
-{
-  if constexpr (LOGN >= 1)
-  {
-    tab[LOGN][kFwd][0] = make_info<LOGN, kFwd, 256>();
-    tab[LOGN][kInv][0] = make_info<LOGN, kInv, 256>();
-    tab[LOGN][kFastconv][0] = make_info<LOGN, kFastconv, 256>();
-    if constexpr (LOGN >= kMin512)
-    {
-      tab[LOGN][kFwd][1] = make_info<LOGN, kFwd, 512>();
-      tab[LOGN][kInv][1] = make_info<LOGN, kInv, 512>();
-      tab[LOGN][kFastconv][1] = make_info<LOGN, kFastconv, 512>();
-    }
-    if constexpr (LOGN >= kMin128 && LOGN <= kMax128)
-    {
-      tab[LOGN][kFwd][2] = make_info<LOGN, kFwd, 128>();
-      tab[LOGN][kInv][2] = make_info<LOGN, kInv, 128>();
-      tab[LOGN][kFastconv][2] = make_info<LOGN, kFastconv, 128>();
-    }
-    if constexpr (LOGN >= kWideLog && LOGN <= kWideMaxLog)
-    {
-      tab[LOGN][kFwd][3] = make_info<LOGN, kFwd, 256, 64>();
-      tab[LOGN][kInv][3] = make_info<LOGN, kInv, 256, 64>();
-      tab[LOGN][kFastconv][3] = make_info<LOGN, kFastconv, 256, 64>();
-    }
-    fill_table<LOGN - 1>(tab);
-  }
-}
-
-static KernelInfo g_table[kMaxLogN + 1][3][kVariants];
+// Kernel table: [mode][logn][variant], variant 0 = 256-thread CTAs, 1 = 512.
+static KernelInfo g_table[3][kMaxLogN + 1][kVariants];
 static std::once_flag g_table_once;
 // Variant chosen per (logn, mode); set by the autotuner through fcb_tune_set.
 static int g_variant[kMaxLogN + 1][3];
@@ -297,7 +251,9 @@ static std::mutex g_variant_mu;
 static void init_table()
 {
   std::call_once(g_table_once, [] {
-    fill_table<kMaxLogN>(g_table);
+    rows_table_fwd(g_table[kFwd]);
+    rows_table_inv(g_table[kInv]);
+    rows_table_conv(g_table[kFastconv]);
     for (int l = 0; l <= kMaxLogN; ++l)
       for (int m = 0; m < 3; ++m)
         // defaults (measured): 4 CTAs of 128 threads per SM for rows of 256 ..
@@ -319,7 +275,7 @@ const KernelInfo *kernel_info(int logn, int mode)
   init_table();
   if (logn < 1 || logn > kMaxLogN || mode < 0 || mode > 2) return nullptr;
   std::lock_guard<std::mutex> lk(g_variant_mu);
-  return &g_table[logn][mode][g_variant[logn][mode]];
+  return &g_table[mode][logn][g_variant[logn][mode]];
 }
 
 // Public tuning values: 128, 256, 512 threads (32 samples per thread), or -256
@@ -338,7 +294,7 @@ const KernelInfo *kernel_variant(int logn, int mode, int threads)
   init_table();
   if (logn < 1 || logn > kMaxLogN || mode < 0 || mode > 2) return nullptr;
   const int v = variant_id(logn, threads);
-  return &g_table[logn][mode][v < 0 ? 0 : v];
+  return &g_table[mode][logn][v < 0 ? 0 : v];
 }
 
 int set_variant(int logn, int mode, int threads)

@@ -66,6 +66,10 @@ struct fcb_plan_s
   const KernelInfo *kchirp = nullptr;          // the kChirpconv kernel for blue_m
   float2 *blue_rep = nullptr;                  // fastconv: replica spectra / n, rows of n
   float2 *blue_buf[2] = {nullptr, nullptr};    // fastconv: rows of n between its two passes
+  // Rows of non-power-of-two length n with small prime factors, and columns of
+  // any such length: the mixed-radix kernel.
+  MixedPlan *mx = nullptr;
+  float2 *mx_rep = nullptr;                    // fastconv: replica table(s), last-stage order
   // Real-input rows of n = rn samples: 1 = real -> complex (n/2 + 1 outputs),
   // 2 = complex -> real.  Even n: a length-n/2 complex plan plus the split /
   // merge step; odd n: a length-n complex plan on expanded rows.
@@ -158,6 +162,8 @@ void plan_free(fcb_plan p)
   }
   cudaFree(p->blue_rep);
   cudaFree(p->chirp_out);
+  mixed_free(p->mx);
+  cudaFree(p->mx_rep);
   plan_free(p->cplx);
   cudaFree(p->rtw);
   cudaFree(p->rbuf);
@@ -197,6 +203,27 @@ int plan_common(fcb_plan p, long long n, long long rows_max, int mode)
     if (rc) return rc;
   }
   return FCB_OK;
+}
+
+// Mixed-radix plan for non-power-of-two n with small prime factors: every such
+// length up to the longest row that fits shared memory.  Against Bluestein's
+// algorithm (two transforms of at least twice the length) it measured 1.3 to 6.7
+// times faster for transforms and 1.5 to 8.5 times for the fast convolution, at
+// 1 to 100000 rows of 18 to 28561 samples; powers of two stay with the row
+// kernels, which are as fast at 1024 and keep two samples per instruction.
+int mixed_setup(fcb_plan p, long long n, long long rows_max, int mode)
+{
+  int rc = check_device();
+  if (rc) return rc;
+  cudaGetDevice(&p->device);
+  p->n = n;
+  p->logn = -1;
+  p->mode = mode;
+  p->rows_max = rows_max;
+  cudaError_t e = cudaStreamCreateWithFlags(&p->own_stream, cudaStreamNonBlocking);
+  if (e != cudaSuccess) return cuda_error(e, "cudaStreamCreate");
+  p->stream = p->own_stream;
+  return mixed_create(n, &p->mx, p->stream);
 }
 
 // Bluestein plan for non-power-of-two n: a chirp and an inner length-m
@@ -655,6 +682,14 @@ int exec_device(fcb_plan p, const float2 *in, long long in_rs, float2 *out, long
                 long long rows, long long row0, cudaStream_t st, int slot)
 {
   if (p->blue_m) return exec_blue(p, in, in_rs, out, out_rs, rows, row0, st, slot);
+  if (p->mx && p->logn < 0)
+  {
+    if (p->mode != kFastconv)
+      return mixed_transform(p->mx, false, in, in_rs, out, out_rs, rows, p->mode == kInv, p->scale, st);
+    const bool per_row = p->rep_rows > 1;
+    return mixed_conv(p->mx, in, in_rs, out, out_rs, rows, p->mx_rep + (per_row ? row0 * p->n : 0), per_row ? p->n : 0,
+                      st);
+  }
   const float4 *rep = p->rep ? p->rep + (p->rep_rows > 1 ? row0 * (p->n > 1 ? p->n / 2 : 1) : 0) : nullptr;
   long long rep_rs = p->rep_rows > 1 ? (p->n > 1 ? p->n / 2 : 1) : 0;
   if (p->logn == 0)
@@ -975,9 +1010,11 @@ int fcb_plan_fftm(long long n, long long rows_max, int exponent, float scale, fc
   if (!p) return set_error(FCB_ERR_NOMEM, "plan allocation");
   p->scale = scale;
   const int mode = exponent == FCB_FORWARD ? kFwd : kInv;
-  int rc = blue_length(n) ? blue_setup(p, n, rows_max, mode, mode == kFwd, mode == kInv)
-                          : plan_common(p, n, rows_max, mode);
-  if (!rc && blue_length(n))
+  const bool mixed = blue_length(n) && mixed_length(n), blue = blue_length(n) && !mixed;
+  int rc = mixed ? mixed_setup(p, n, rows_max, mode)
+         : blue ? blue_setup(p, n, rows_max, mode, mode == kFwd, mode == kInv)
+                : plan_common(p, n, rows_max, mode);
+  if (!rc && blue)
   {
     // the output multiplier of a Bluestein row: the chirp times the scale
     cudaError_t e = cudaMalloc(&p->chirp_out, sizeof(float2) * (size_t)n);
@@ -1009,8 +1046,9 @@ int fcb_plan_fastconv(long long n, long long rows_max, const fcb_cf32 *replica, 
   if (where != FCB_HOST && where != FCB_DEVICE) return set_error(FCB_ERR_INVALID, "bad location");
   fcb_plan p = new (std::nothrow) fcb_plan_s;
   if (!p) return set_error(FCB_ERR_NOMEM, "plan allocation");
-  const bool blue = blue_length(n);
-  int rc = blue ? blue_setup(p, n, rows_max, kFastconv, true, true) : plan_common(p, n, rows_max, kFastconv);
+  const bool mixed = blue_length(n) && mixed_length(n), blue = blue_length(n) && !mixed;
+  int rc = mixed ? mixed_setup(p, n, rows_max, kFastconv)
+         : blue ? blue_setup(p, n, rows_max, kFastconv, true, true) : plan_common(p, n, rows_max, kFastconv);
   float2 *spec = nullptr, *tmp = nullptr;
   if (!rc)
   {
@@ -1033,7 +1071,14 @@ int fcb_plan_fastconv(long long n, long long rows_max, const fcb_cf32 *replica, 
         rc = replica_spectrum_dev(spec + r * n, n, replica_kind == FCB_REPLICA_TIME_MATCHED, tmp + r * n, p->stream);
       if (!rc) std::swap(spec, tmp);
     }
-    if (!rc && blue)
+    if (!rc && mixed)
+    {
+      p->rep_rows = replica_rows;
+      e = cudaMalloc(&p->mx_rep, bytes);
+      if (e != cudaSuccess) rc = set_error(FCB_ERR_NOMEM, "replica table: %s", cudaGetErrorString(e));
+      if (!rc) rc = mixed_replica(p->mx, spec, n, replica_rows, (float)(1.0 / (double)n), p->mx_rep, p->stream);
+    }
+    else if (!rc && blue)
     {
       // R / n per row; 1/n is the inverse FFT's normalisation
       p->rep_rows = replica_rows;
@@ -1165,6 +1210,12 @@ int fcb_plan_info(fcb_plan p, long long *n, int *cluster_ctas, int *rows_per_cta
   // Bluestein and real-input plans report the kernel of their power-of-two work rows
   fcb_plan q = p->cplx ? p->cplx : p;
   const KernelInfo *k = q->k ? q->k : q->inner[0] ? q->inner[0]->k : q->inner[1] ? q->inner[1]->k : nullptr;
+  if (!k && q->mx)
+  {
+    mixed_info(q->mx, q->rows_max, rows_per_cta, smem_bytes, threads);
+    if (cluster_ctas) *cluster_ctas = 1;
+    return FCB_OK;
+  }
   if (threads) *threads = k ? k->threads : 0;
   if (cluster_ctas) *cluster_ctas = k ? k->cluster : 1;
   if (rows_per_cta) *rows_per_cta = k ? k->rows_per_cta : 1;

@@ -38,6 +38,10 @@ constexpr int kWideMaxLog = 15;  // and 32768 on clusters of two CTAs
 // wide one.  Its public tuning value is -256.
 constexpr int kVariants = 4;
 
+// Entries [logn][variant] of one mode (fcb_rows_*.cu)
+void rows_table_fwd(KernelInfo (*tab)[kVariants]);
+void rows_table_inv(KernelInfo (*tab)[kVariants]);
+void rows_table_conv(KernelInfo (*tab)[kVariants]);
 const KernelInfo *kernel_info(int logn, int mode);
 // Fused kernel with element-wise multipliers (kChirpconv, fcb_bluestein.cu)
 // for work rows of 2^logn samples, in the same variant as `like` (whose
@@ -66,6 +70,27 @@ int launch_scale_rows(const float2 *in, long long in_rs, float2 *out, long long 
 // length N, computed through power-of-two work rows of M >= 2N - 1 samples.
 int bluestein_tables(long long N, long long M, int sign, float2 **chirp, float2 **spectrum, cudaStream_t st);
 int scale_copy(const float2 *in, float2 *out, long long total, float s, cudaStream_t st);
+
+// Mixed-radix plans (fcb_mixed.cu): lengths whose prime factors are at most 13,
+// one row in shared memory.  Device tables only; a plan may be used from several
+// streams and threads at once.
+struct MixedPlan;
+bool mixed_length(long long n);
+int mixed_create(long long n, MixedPlan **out, cudaStream_t st);
+void mixed_free(MixedPlan *p);
+void mixed_info(const MixedPlan *p, long long rows, int *rows_per_cta, int *smem, int *threads);
+// replica table: rows spectra of n values, times scale (the 1/n belongs in it), into rows * n values
+int mixed_replica(const MixedPlan *p, const float2 *spec, long long spec_rs, long long rows, float scale, float2 *rep,
+                  cudaStream_t st);
+// `count` rows (or, with columns, columns) of a matrix whose rows are in_ld / out_ld apart
+int mixed_transform(MixedPlan *p, bool columns, const float2 *in, long long in_ld, float2 *out, long long out_ld,
+                    long long count, bool inverse, float scale, cudaStream_t st);
+int mixed_conv(MixedPlan *p, const float2 *in, long long in_rs, float2 *out, long long out_rs, long long rows,
+               const float2 *rep, long long rep_rs, cudaStream_t st);
+// Bluestein pass over rows of n samples in the plan's work length (>= 2 n - 1)
+int mixed_chirp(MixedPlan *p, const float2 *in, long long in_rs, float2 *out, long long out_rs, long long rows,
+                long long n, const float2 *cin, long long cin_rs, const float2 *cout, const float2 *rep,
+                cudaStream_t st);
 
 // Real-input row FFTs (fcb_real.cu).
 int real_twiddles(long long n, long long count, float2 **out, cudaStream_t st);

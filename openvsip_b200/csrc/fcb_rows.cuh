@@ -1,0 +1,39 @@
+// Kernel table entries of the row kernels (the variants of every length).  Each
+// mode is instantiated in a translation unit of its own, so that they compile
+// side by side.
+#pragma once
+
+#include "fcb_engine.cuh"
+#include "fcb_internal.h"
+
+namespace fcb {
+
+template <int LOGN, int MODE, int T, int EPTW = 32>
+KernelInfo rows_info()
+{
+  using S = Sched<LOGN, T, EPTW>;
+  KernelInfo k;
+  k.fn = (const void *)&rows_kernel<LOGN, MODE, T, EPTW>;
+  k.ept = EPTW;
+  k.threads = T;
+  k.cluster = S::CS;
+  k.rows_per_cta = S::ROWS;
+  k.smem = S::SMEM;
+  k.tw_bytes = S::tw_bytes();
+  return k;
+}
+
+template <int MODE, int LOGN = kMaxLogN>
+void fill_rows_table(KernelInfo (*tab)[kVariants])
+{
+  if constexpr (LOGN >= 1)
+  {
+    tab[LOGN][0] = rows_info<LOGN, MODE, 256>();
+    if constexpr (LOGN >= kMin512) tab[LOGN][1] = rows_info<LOGN, MODE, 512>();
+    if constexpr (LOGN >= kMin128 && LOGN <= kMax128) tab[LOGN][2] = rows_info<LOGN, MODE, 128>();
+    if constexpr (LOGN >= kWideLog && LOGN <= kWideMaxLog) tab[LOGN][3] = rows_info<LOGN, MODE, 256, 64>();
+    fill_rows_table<MODE, LOGN - 1>(tab);
+  }
+}
+
+}  // namespace fcb
