@@ -94,7 +94,8 @@ FCB_API const char *fcb_version(void);
 FCB_API int fcb_init(int device);
 /* 1 if n is a supported row length for Fftm and fast-convolution plans: any
  * length in [1, 32768], or a power of two up to 65536.  Powers of two run as
- * one fused pass; other lengths by Bluestein's chirp-z algorithm: the fused
+ * one fused pass, and so do lengths up to 28672 with no prime factor above 13
+ * (mixed radix); other lengths by Bluestein's chirp-z algorithm: the fused
  * kernel runs on work rows of the next power of two >= 2n - 1 samples and
  * applies the chirps, the zero padding and the truncation to n samples on its
  * own loads and stores (one pass per transform).  The reference's FFTW
@@ -179,6 +180,18 @@ FCB_API int fcb_exec(fcb_plan plan, const fcb_cf32 *in, long long in_rs, fcb_cf3
  * Fftm calls are synchronous).  With where = FCB_DEVICE it is fcb_exec. */
 FCB_API int fcb_exec_async(fcb_plan plan, const fcb_cf32 *in, long long in_rs, fcb_cf32 *out,
                            long long out_rs, long long rows, int where);
+
+/* Column transforms without transposing: an n x cols matrix (row strides in_rs /
+ * out_rs >= cols), each of its columns transformed; in place with equal strides
+ * is allowed.  A host call returns with the output written.  Replaces fftm_backend<..., 1, D>
+ * over columns (src/ovxx/fftw/fftw.cpp:904-977).  fcb_supported_cols says
+ * which n have such a kernel; fcb_plan_fftm_cols makes a plan that serves
+ * fcb_exec_cols (up to cols_max columns) and, over rows of n, fcb_exec. */
+FCB_API int fcb_supported_cols(long long n);
+FCB_API int fcb_plan_fftm_cols(long long n, long long cols_max, int exponent, float scale,
+                               fcb_plan *plan);
+FCB_API int fcb_exec_cols(fcb_plan plan, const fcb_cf32 *in, long long in_rs, fcb_cf32 *out,
+                          long long out_rs, long long cols, int where);
 
 /* Queue the plan's device work on a caller-owned cudaStream_t (NULL is the
  * CUDA default stream).  A new plan uses a private non-blocking stream. */

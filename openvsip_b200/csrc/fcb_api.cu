@@ -70,6 +70,8 @@ struct fcb_plan_s
   // any such length: the mixed-radix kernel.
   MixedPlan *mx = nullptr;
   float2 *mx_rep = nullptr;                    // fastconv: replica table(s), last-stage order
+  float2 *cstage = nullptr;                    // host column calls: device copy of a block of columns
+  long long cstage_cols = 0;
   // Real-input rows of n = rn samples: 1 = real -> complex (n/2 + 1 outputs),
   // 2 = complex -> real.  Even n: a length-n/2 complex plan plus the split /
   // merge step; odd n: a length-n complex plan on expanded rows.
@@ -164,6 +166,7 @@ void plan_free(fcb_plan p)
   cudaFree(p->chirp_out);
   mixed_free(p->mx);
   cudaFree(p->mx_rep);
+  cudaFree(p->cstage);
   plan_free(p->cplx);
   cudaFree(p->rtw);
   cudaFree(p->rbuf);
@@ -1029,6 +1032,70 @@ int fcb_plan_fftm(long long n, long long rows_max, int exponent, float scale, fc
   if (rc) { plan_free(p); return rc; }
   *plan = p;
   return FCB_OK;
+}
+
+int fcb_supported_cols(long long n) { return mixed_columns(n); }
+
+int fcb_plan_fftm_cols(long long n, long long cols_max, int exponent, float scale, fcb_plan *plan)
+{
+  int rc = fcb_plan_fftm(n, cols_max, exponent, scale, plan);
+  if (rc) return rc;
+  fcb_plan p = *plan;
+  if (!p->mx && fcb_supported_cols(n))
+  {
+    DeviceGuard g(p->device);
+    rc = mixed_create(n, &p->mx, p->stream);
+    cudaError_t e = cudaSuccess;
+    if (!rc && (e = cudaStreamSynchronize(p->stream)) != cudaSuccess) rc = cuda_error(e, "plan tables");
+    if (rc)
+    {
+      plan_free(p);
+      *plan = nullptr;
+    }
+  }
+  return rc;
+}
+
+int fcb_exec_cols(fcb_plan p, const fcb_cf32 *in, long long in_rs, fcb_cf32 *out, long long out_rs, long long cols,
+                  int where)
+{
+  if (!p) return set_error(FCB_ERR_INVALID, "plan is NULL");
+  if (!p->mx || p->mode == kFastconv || !fcb_supported_cols(p->n))
+    return set_error(FCB_ERR_UNSUPPORTED, "not a plan of fcb_plan_fftm_cols with a column kernel");
+  if (cols < 0 || cols > p->rows_max) return set_error(FCB_ERR_INVALID, "cols %lld outside [0, %lld]", cols, p->rows_max);
+  if (cols == 0) return FCB_OK;
+  if (!in || !out) return set_error(FCB_ERR_INVALID, "NULL data pointer");
+  if (in_rs < cols || out_rs < cols) return set_error(FCB_ERR_INVALID, "row stride smaller than the row length");
+  if ((const void *)in == (const void *)out && in_rs != out_rs)
+    return set_error(FCB_ERR_INVALID, "in-place call with different row strides");
+  if (where != FCB_HOST && where != FCB_DEVICE) return set_error(FCB_ERR_INVALID, "bad location");
+  DeviceGuard g(p->device);
+  const float2 *i2 = reinterpret_cast<const float2 *>(in);
+  float2 *o2 = reinterpret_cast<float2 *>(out);
+  if (where == FCB_DEVICE)
+    return mixed_transform(p->mx, true, i2, in_rs, o2, out_rs, cols, p->mode == kInv, p->scale, p->stream);
+  // host columns: blocks of them through one device buffer
+  const long long n = p->n, chunk = std::min(cols, std::max<long long>(1, (long long)(4 * stage_bytes()) / (8 * n)));
+  if (p->cstage_cols < chunk)
+  {
+    cudaFree(p->cstage);
+    p->cstage = nullptr;
+    p->cstage_cols = 0;
+    const cudaError_t e = cudaMalloc(&p->cstage, sizeof(float2) * (size_t)(chunk * n));
+    if (e != cudaSuccess) return set_error(FCB_ERR_NOMEM, "staging buffer: %s", cudaGetErrorString(e));
+    p->cstage_cols = chunk;
+  }
+  int rc = FCB_OK;
+  for (long long c0 = 0; !rc && c0 < cols; c0 += chunk)
+  {
+    const long long nc = std::min(chunk, cols - c0);
+    const size_t rb = sizeof(float2) * (size_t)nc;
+    rc = copy_h2d(p, p->cstage, rb, i2 + c0, sizeof(float2) * (size_t)in_rs, rb, (size_t)n, p->stream);
+    if (!rc)
+      rc = mixed_transform(p->mx, true, p->cstage, nc, p->cstage, nc, nc, p->mode == kInv, p->scale, p->stream);
+    if (!rc) rc = copy_d2h(p, o2 + c0, sizeof(float2) * (size_t)out_rs, p->cstage, rb, rb, (size_t)n, p->stream);
+  }
+  return host_done(p, rc, "fcb_exec_cols (host)");
 }
 
 int fcb_plan_fastconv(long long n, long long rows_max, const fcb_cf32 *replica, long long replica_rows,

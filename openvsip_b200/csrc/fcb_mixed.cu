@@ -31,7 +31,9 @@
 // per call, against two Bluestein transforms in the row kernels: transform at
 // 480 / 756 / 1000 / 1144 / 3000 samples 43.7 / 52.7 / 43.4 / 65.6 / 69.6 us ->
 // 20.5 / 20.5 / 22.6 / 18.9 / 23.1 us (67 MB: 2.9 - 3.6 TB/s); fast convolution
-// at 480 / 1144 / 3000: 88 / 134 / 131 us -> 28.7 / 30.7 / 38.7 us.
+// at 480 / 1144 / 3000: 88 / 134 / 131 us -> 28.7 / 30.7 / 38.7 us.  Columns,
+// against transposing copies around the row kernels: 1144 columns of 756 24.4 ->
+// 6.0 us, 1024 of 4096 61 -> 19 us, 4096 of 4096 219 -> 104 us.
 #include "fcb200.h"
 #include "fcb_internal.h"
 
@@ -50,6 +52,10 @@ namespace {
 constexpr int kMrStages = 8;
 constexpr int kMrSmem = 227 * 1024;  // shared memory of one CTA, and of an SM
 constexpr int kMrMaxN = 28 * 1024;   // longest row that fits
+// Longest column: two side by side fit.  Measured against transposing into rows and back:
+// 8192 columns of 512 45 against 62 us; one column per CTA (16384 columns of 256, 8-byte
+// accesses) 80 against 67 us.
+constexpr int kMrMaxCol = kMrMaxN / 2;
 
 struct MrStage
 {
@@ -662,6 +668,8 @@ int mixed_launch(MixedPlan *p, int kind, bool col, MrArgs &a, cudaStream_t st)
 }
 
 }  // namespace
+
+bool mixed_columns(long long n) { return n <= kMrMaxCol && mixed_length(n); }
 
 bool mixed_length(long long n)
 {

@@ -129,7 +129,8 @@ def _transposed(x):
     """Contiguous transpose: the column-major copy the reference's DDA layer makes
     for a column-axis Fftm (query_layout asks for tuple<1,0,2>)."""
     if _is_torch(x):
-        return x.t().contiguous()
+        # a lazy conjugate would survive contiguous() where no copy is needed (one column)
+        return x.t().resolve_conj().resolve_neg().contiguous()
     return np.ascontiguousarray(x.T)
 
 
@@ -139,6 +140,34 @@ def _put_transposed(out, yt):
     else:
         out[...] = yt.T
     return out
+
+
+def _plain_matrix(x, writable: bool):
+    """(pointer, rows, cols, row stride, where) of a complex64 matrix with
+    unit-stride rows that its memory holds as they are (no lazy conjugate, no
+    rows on top of each other); None for anything else."""
+    if type(x) is np.ndarray:
+        if (x.dtype != np.complex64 or x.ndim != 2 or x.size == 0 or x.strides[1] != 8 or x.strides[0] % 8
+                or x.strides[0] < 8 * x.shape[1] or writable and not x.flags.writeable):
+            return None
+        return x.ctypes.data, x.shape[0], x.shape[1], x.strides[0] // 8, _lib.FCB_HOST
+    if not _is_torch(x):
+        return None
+    t = _torch_mod()
+    if not (type(x) is t.Tensor and x.dtype is t.complex64 and x.is_cuda and x.dim() == 2 and x.numel() > 0):
+        return None
+    rs, cs = x.stride()
+    if cs != 1 or rs < x.shape[1] or x.is_conj() or x.is_neg() or writable and x.requires_grad:
+        return None
+    return x.data_ptr(), x.shape[0], x.shape[1], rs, _lib.FCB_DEVICE
+
+
+def _same_or_apart(a, b) -> bool:
+    """Two matrices of _plain_matrix are the same one, or share no memory."""
+    if a[0] == b[0]:
+        return a[3] == b[3]
+    span = lambda m: 8 * ((m[1] - 1) * m[3] + m[2])  # noqa: E731
+    return a[0] + span(a) <= b[0] or b[0] + span(b) <= a[0]
 
 
 class _Plan:
@@ -213,9 +242,11 @@ class Fftm(_Plan):
     """Multiple FFT on the GPU (vsip::Fftm<C, C, A, D, R>).
 
     axis=row (default) transforms each of the `rows` rows of length `cols`;
-    axis=col transforms each of the `cols` columns of length `rows`.  Column
-    data is transposed into contiguous rows and back around the row kernel, as
-    the reference's DDA layer does for its FFTW backend."""
+    axis=col transforms each of the `cols` columns of length `rows`.  Columns
+    whose length has a column kernel (fcb_supported_cols) are transformed where
+    they are; other column data is transposed into contiguous
+    rows and back around the row kernel, as the reference's DDA layer does for
+    its FFTW backend."""
 
     def __init__(self, rows: int, cols: int, direction: int = fft_fwd, scale: float = 1.0, axis: int = row):
         self.rows, self.cols = int(rows), int(cols)
@@ -224,22 +255,34 @@ class Fftm(_Plan):
         self.scale = float(scale)
         n, count = (self.cols, self.rows) if self.axis == row else (self.rows, self.cols)
         h = ctypes.c_void_p()
-        check(lib().fcb_plan_fftm(n, count, self.exponent, self.scale, ctypes.byref(h)))
+        plan = lib().fcb_plan_fftm if self.axis == row else lib().fcb_plan_fftm_cols
+        check(plan(n, count, self.exponent, self.scale, ctypes.byref(h)))
         self._handle = h
         self._n = n
+        self._col_kernel = self.axis == col and bool(lib().fcb_supported_cols(n))
 
     def __call__(self, inp, out=None):
         """By reference: ``fftm(in, out)``; ``fftm(in)`` returns a new result (by value)."""
         if out is None:
             out = _empty_like(inp)
         if self.axis == col:
-            return _put_transposed(out, self._rows(_transposed(inp)))
+            return self._columns(inp, out)
         return self._exec(inp, out)
 
     def in_place(self, inout):
         if self.axis == col:
-            return _put_transposed(inout, self._rows(_transposed(inout)))
+            return self._columns(inout, inout)
         return self._exec(inout, inout)
+
+    def _columns(self, inp, out):
+        a = _plain_matrix(inp, False) if self._col_kernel else None
+        b = _plain_matrix(out, True) if a else None
+        if not (a and b and a[1:3] == b[1:3] and a[1] == self._n and a[2] <= self.cols and a[4] == b[4]
+                and _same_or_apart(a, b)):
+            return _put_transposed(out, self._rows(_transposed(inp)))
+        self._bind_stream(a[4])
+        check(lib().fcb_exec_cols(self._handle, a[0], a[3], b[0], b[3], a[2], a[4]))
+        return out
 
     def _rows(self, xt):
         return self._exec(xt, _empty_like(xt))

@@ -2,12 +2,13 @@
 most 13, up to 28672 samples) against the FP64 oracle: relative L2 <= 2e-6, the
 bar of the other row kernels.  The sizes are where its plan changes: one to six
 stages, every radix, several rows per CTA with a partial last one, the longest
-rows (512-thread CTAs)."""
+rows (512-thread CTAs); columns likewise, and the forms of a matrix that go
+through rows instead."""
 import numpy as np
 import pytest
 
 from conftest import crandn
-from openvsip_b200 import Fastconv, Fftm, fft_fwd, fft_inv
+from openvsip_b200 import FcbError, Fastconv, Fftm, col, fft_fwd, fft_inv
 
 pytestmark = pytest.mark.gpu
 RTOL = 2e-6
@@ -46,3 +47,44 @@ def test_fastconv_vector_and_matrix(oracle, rows, n):
     for w in (crandn(rng, (n,)), crandn(rng, (rows, n))):
         y = Fastconv(w, rows)(torch.from_numpy(x).cuda())
         assert oracle.rel_l2(y.cpu().numpy(), oracle.fastconv(x, w)) <= RTOL
+
+
+#       one column, one stage, partial last CTA, ragged, two columns per CTA, the longest, longer: through rows
+COLUMNS = [(13, 1), (2, 70), (756, 45), (1000, 67), (4096, 9), (8192, 5), (14336, 3), (16384, 3), (67, 5)]
+
+
+@pytest.mark.parametrize("n,m", COLUMNS)
+@pytest.mark.parametrize("direction", [fft_fwd, fft_inv])
+def test_columns_host_device_views_and_in_place(n, m, direction):
+    import torch
+    rng = np.random.default_rng(n + m)
+    big = crandn(rng, (n, m + 6))
+    x = big[:, 1:m + 1]
+    scale = 0.25 if direction == fft_fwd else 1.0 / n
+    x64 = x.astype(np.complex128)
+    want = scale * (np.fft.fft(x64, axis=0) if direction == fft_fwd else n * np.fft.ifft(x64, axis=0))
+    rel = lambda y: np.linalg.norm(y - want) / np.linalg.norm(want)  # noqa: E731
+    f = Fftm(n, m, direction, scale, axis=col)
+    host = f(x)
+    assert rel(host) <= RTOL
+    dbig = torch.from_numpy(big.copy()).cuda()
+    dx = dbig[:, 1:m + 1]
+    out = torch.zeros(n, m + 4, dtype=torch.complex64, device="cuda")
+    f(dx, out[:, 3:m + 3])
+    assert np.array_equal(out[:, 3:m + 3].cpu().numpy(), host)
+    assert not out[:, :3].any() and not out[:, m + 3:].any()
+    # inputs that no column kernel takes as they are: a lazy conjugate, a transposed
+    # view, an output that overlaps the input
+    assert rel(f(torch.from_numpy(np.ascontiguousarray(x).conj()).cuda().conj()).cpu().numpy()) <= RTOL
+    assert rel(f(torch.from_numpy(np.ascontiguousarray(x.T)).cuda().t()).cpu().numpy()) <= RTOL
+    over = dbig.clone()
+    assert rel(f(over[:, 1:m + 1], over[:, 2:m + 2]).cpu().numpy()) <= RTOL
+    h = np.ascontiguousarray(x)
+    assert np.array_equal(f.in_place(h), host)
+    f.in_place(dx)
+    assert np.array_equal(dx.cpu().numpy(), host)
+    assert torch.equal(dbig[:, m + 1:].cpu(), torch.from_numpy(big[:, m + 1:].copy()))  # neighbours untouched
+    if m > 2:  # fewer columns than planned
+        assert np.array_equal(f(np.ascontiguousarray(x[:, :2])), host[:, :2])
+    with pytest.raises(FcbError):
+        f(crandn(rng, (n, m + 1)))
