@@ -297,6 +297,19 @@ const KernelInfo *kernel_variant(int logn, int mode, int threads)
   return &g_table[mode][logn][v < 0 ? 0 : v];
 }
 
+const KernelInfo *real_kernel(int logn, bool inverse, const KernelInfo *like)
+{
+  static KernelInfo tab[2][kMaxLogN + 1][kVariants];
+  static std::once_flag once;
+  std::call_once(once, [] {
+    rows_table_r2c(tab[0]);
+    rows_table_c2r(tab[1]);
+  });
+  if (logn < 1 || logn > kMaxLogN || !like) return nullptr;
+  const int v = variant_id(logn, like->ept == 64 ? -like->threads : like->threads);
+  return v < 0 || !tab[inverse][logn][v].fn ? nullptr : &tab[inverse][logn][v];
+}
+
 int set_variant(int logn, int mode, int threads)
 {
   init_table();

@@ -79,6 +79,8 @@ struct fcb_plan_s
   long long rn = 0;
   fcb_plan cplx = nullptr;
   float2 *rtw = nullptr;               // W_n^k, k = 0 .. n/2 (even n)
+  const KernelInfo *kreal = nullptr;   // n/2 a power of two: the row kernel with the split / merge step, if any
+  float4 *rtw4 = nullptr;              // real -> complex there: pairs of W_n^k
   float2 *rbuf = nullptr;              // work rows (odd n, or unaligned rows)
   long long rbuf_rows = 0, rbuf_cols = 0;
   void *rstage[2] = {nullptr, nullptr};  // host calls: device copies of in / out
@@ -169,6 +171,7 @@ void plan_free(fcb_plan p)
   cudaFree(p->cstage);
   plan_free(p->cplx);
   cudaFree(p->rtw);
+  cudaFree(p->rtw4);
   cudaFree(p->rbuf);
   cudaFree(p->rstage[0]);
   cudaFree(p->rstage[1]);
@@ -338,6 +341,26 @@ int ensure_rbuf(fcb_plan p, long long cols)
   return FCB_OK;
 }
 
+// Real rows of n = 2^k samples through the row kernel of n/2: the real side as
+// complex rows of n/2, the other as rows of n/2 + 1.
+int exec_real_rows(fcb_plan p, const float2 *in, long long in_rs, float2 *out, long long out_rs, long long rows,
+                   cudaStream_t st)
+{
+  RowArgs a = {};
+  a.in = in;
+  a.in_rs = in_rs;
+  a.out = out;
+  a.out_rs = out_rs;
+  a.rows = rows;
+  a.tw = a.twi = p->cplx->tw;
+  a.rep = p->rtw4;
+  a.cin = p->rtw;
+  a.scale = p->scale;
+  a.vec_out = (reinterpret_cast<uintptr_t>(out) % 16 == 0) && (out_rs % 2 == 0 || rows == 1);
+  a.ahead = -1;
+  return launch_rows(p->kreal, rows, a, st);
+}
+
 // Real-input rows on device pointers, stream st.  in / out: float rows of n
 // (real side) or complex rows of n/2 + 1 (spectrum side); strides in elements.
 int exec_real_device(fcb_plan p, const void *in, long long in_rs, void *out, long long out_rs, long long rows,
@@ -369,6 +392,11 @@ int exec_real_device(fcb_plan p, const void *in, long long in_rs, void *out, lon
           z = p->rbuf;
           z_rs = m;
         }
+        if (p->kreal)
+        {
+          rc = exec_real_rows(p, z, z_rs, y + r0 * out_rs, out_rs, nr, st);
+          continue;
+        }
         rc = exec_device(p->cplx, z, z_rs, y + r0 * out_rs, out_rs, nr, 0, st);
         if (!rc) rc = r2c_post(y + r0 * out_rs, out_rs, m, nr, p->rtw, p->scale, st);
       }
@@ -385,8 +413,13 @@ int exec_real_device(fcb_plan p, const void *in, long long in_rs, void *out, lon
         const long long nr = std::min(chunk, rows - r0);
         float2 *z = direct ? reinterpret_cast<float2 *>(y + r0 * out_rs) : p->rbuf;
         const long long z_rs = direct ? (rows == 1 ? m : out_rs / 2) : m;
-        rc = c2r_pre(x + r0 * in_rs, in_rs, z, z_rs, m, nr, p->rtw, st);
-        if (!rc) rc = exec_device(p->cplx, z, z_rs, z, z_rs, nr, 0, st);
+        if (p->kreal)
+          rc = exec_real_rows(p, x + r0 * in_rs, in_rs, z, z_rs, nr, st);
+        else
+        {
+          rc = c2r_pre(x + r0 * in_rs, in_rs, z, z_rs, m, nr, p->rtw, st);
+          if (!rc) rc = exec_device(p->cplx, z, z_rs, z, z_rs, nr, 0, st);
+        }
         if (!rc && !direct)
         {
           cudaError_t e = cudaMemcpy2DAsync(y + r0 * out_rs, sizeof(float) * (size_t)out_rs, p->rbuf,
@@ -1325,6 +1358,12 @@ int fcb_plan_fftm_real(long long n, long long rows_max, int exponent, float scal
     rc = fcb_plan_fftm(even ? n / 2 : n, std::max<long long>(rows_max, 1), exponent,
                        (even && p->real == 1) ? 1.f : scale, &p->cplx);
   if (!rc && even) rc = real_twiddles(n, n / 2 + 1, &p->rtw, p->stream);
+  if (!rc && even && p->cplx->k)
+  {
+    p->kreal = real_kernel(p->cplx->logn, p->real == 2, p->cplx->k);
+    if (p->kreal) rc = prepare_kernel(p->kreal);
+    if (!rc && p->kreal && p->real == 1) rc = real_twiddle_pairs(n, &p->rtw4, p->stream);
+  }
   if (!rc && (e = cudaStreamSynchronize(p->stream)) != cudaSuccess) rc = cuda_error(e, "real-FFT tables");
   if (rc) { plan_free(p); return rc; }
   *plan = p;

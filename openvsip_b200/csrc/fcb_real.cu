@@ -13,7 +13,9 @@
 // O'[k] = (X[k] - conj X[m-k]) W_n^-k, then an unnormalised inverse length-m
 // FFT gives x[2j] + i x[2j+1].  As FFTW's c2r does, the imaginary parts of
 // X[0] and X[m] are ignored (the input is taken as the half spectrum of a real
-// signal).
+// signal).  For m a power of two the split and the merge are part of the row
+// kernel (its kR2C and kC2R modes: one pass over the rows); for other m, and for
+// the split of rows that span a cluster, they are passes of their own, below.
 //
 // Odd n: rows go through the length-n complex FFT (Bluestein) with a zero
 // imaginary part (forward) or the full Hermitian spectrum (inverse).
@@ -46,6 +48,19 @@ __global__ void real_tw_kernel(float2 *w, long long n, long long count)
   double s, c;
   sincospi(-2.0 * (double)k / (double)n, &s, &c);
   w[k] = make_float2((float)c, (float)s);
+}
+
+// w[m] = (W_n^2m, W_n^(2m+1)) and w[n/4 + m] = (W_n^(2m+1), W_n^(2m+2)), as
+// (re, re, im, im), m < n / 4.
+__global__ void real_tw_pair_kernel(float4 *w, long long n)
+{
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n / 2) return;
+  const long long k = i < n / 4 ? 2 * i : 2 * (i - n / 4) + 1;
+  double s0, c0, s1, c1;
+  sincospi(-2.0 * (double)k / (double)n, &s0, &c0);
+  sincospi(-2.0 * (double)(k + 1) / (double)n, &s1, &c1);
+  w[i] = make_float4((float)c0, (float)c1, (float)s0, (float)s1);
 }
 
 // X[j] = E_j + W^j O_j from Z[j] and Z[m - j], for j = k and j = m - k, in place.
@@ -154,6 +169,18 @@ int real_twiddles(long long n, long long count, float2 **out, cudaStream_t st)
   cudaError_t e = cudaMalloc(&w, sizeof(float2) * (size_t)count);
   if (e != cudaSuccess) return set_error(FCB_ERR_NOMEM, "real-FFT twiddles: %s", cudaGetErrorString(e));
   real_tw_kernel<<<(unsigned)((count + 255) / 256), 256, 0, st>>>(w, n, count);
+  int rc = launched("real-FFT twiddles");
+  if (rc) { cudaFree(w); return rc; }
+  *out = w;
+  return FCB_OK;
+}
+
+int real_twiddle_pairs(long long n, float4 **out, cudaStream_t st)
+{
+  float4 *w = nullptr;
+  cudaError_t e = cudaMalloc(&w, sizeof(float4) * (size_t)(n / 2));
+  if (e != cudaSuccess) return set_error(FCB_ERR_NOMEM, "real-FFT twiddles: %s", cudaGetErrorString(e));
+  real_tw_pair_kernel<<<(unsigned)((n / 2 + 255) / 256), 256, 0, st>>>(w, n);
   int rc = launched("real-FFT twiddles");
   if (rc) { cudaFree(w); return rc; }
   *out = w;

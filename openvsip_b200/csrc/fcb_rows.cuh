@@ -13,7 +13,8 @@ KernelInfo rows_info()
 {
   using S = Sched<LOGN, T, EPTW>;
   KernelInfo k;
-  k.fn = (const void *)&rows_kernel<LOGN, MODE, T, EPTW>;
+  // the split of real rows has no cluster form (entry left empty)
+  if constexpr (MODE != kR2C || S::CS == 1) k.fn = (const void *)&rows_kernel<LOGN, MODE, T, EPTW>;
   k.ept = EPTW;
   k.threads = T;
   k.cluster = S::CS;
