@@ -22,7 +22,7 @@ FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler", 
          f"-I{os.path.join(ROOT, 'include')}", f"-I{CSRC}"]
 
 SOURCES = ["fcb_rows_conv.cu", "fcb_rows_fwd.cu", "fcb_rows_inv.cu", "fcb_rows_r2c.cu",
-           "fcb_rows_c2r.cu", "fcb_batch.cu", "fcb_mixed.cu", "fcb200.cu",
+           "fcb_rows_c2r.cu", "fcb_rows_cross.cu", "fcb_batch.cu", "fcb_mixed.cu", "fcb200.cu",
            "fcb_api.cu", "fcb_bluestein.cu", "fcb_real.cu", "fcb_hostcopy.cu"]
 
 # The mixed-radix kernels dominate the build when compiled one after another.

@@ -48,6 +48,11 @@ struct fcb_plan_s
   float4 *twc = nullptr;
   float2 *scratch = nullptr;
   float2 *stage2d_in = nullptr, *stage2d_out = nullptr;
+  // Where the row pass can take the columns' first stage along: that row kernel,
+  // and the mixed-radix plan of the rest of the columns.
+  const CrossKernel *kx = nullptr;
+  MixedPlan *mxc = nullptr;
+  float2 *twx = nullptr;           // W^k of the column length
   // 2-D FFT of other sizes (any dimensions the row plans support): a row plan
   // of length cols, a transpose, a row plan of length rows on the transposed
   // matrix, and a transpose back; scratch2 holds the transposed matrix.
@@ -102,6 +107,14 @@ constexpr long long kMaxBlueN = 1LL << (kMaxLogN - 1);
 constexpr long long kBlueChunkSamples = 1LL << 25;  // work buffer: 256 MiB at most
 
 bool blue_length(long long n) { return n > 0 && n <= kMaxBlueN && (n & (n - 1)) != 0; }
+
+// 2-D transforms whose row pass takes the columns' first stage along.  Longest
+// columns left to the second pass: four of them (a 32-byte sector of each row) fit
+// its CTA.  Smallest matrix: against two transposing passes 4096 x 4096 measured
+// 179 -> 144 us, 8192 x 8192 917 -> 709, 1024 x 8192 106 -> 77, 2048 x 2048 45.4 ->
+// 40.4, but 1024 x 1024 14.9 -> 16.4 and 512 x 512 11.9 -> 12.2 us (the second
+// pass's stages take longer than one more row pass when both are a single wave).
+constexpr long long kCrossMaxRest = 4096, kCrossMinSamples = 1LL << 21;
 
 #define FCB_LENGTH_RULE "any length in [1, 32768], or a power of two up to 65536"
 
@@ -167,6 +180,8 @@ void plan_free(fcb_plan p)
   cudaFree(p->blue_rep);
   cudaFree(p->chirp_out);
   mixed_free(p->mx);
+  mixed_free(p->mxc);
+  cudaFree(p->twx);
   cudaFree(p->mx_rep);
   cudaFree(p->cstage);
   plan_free(p->cplx);
@@ -694,6 +709,24 @@ int exec_2d(fcb_plan p, const float2 *in, long long in_rs, float2 *out, long lon
   RowArgs a = {};
   a.in = in;
   a.in_rs = in_rs;
+  if (p->kx)
+  {
+    // rows and the first stage of the columns, then the rest of the columns:
+    // scratch row cross q + n' holds output q of that stage, whose remaining
+    // transform over n' gives the rows q + radix k
+    const long long R = p->rows2d, C = p->cols2d, G = p->kx->radix, cross = R / G;
+    a.out = p->scratch;
+    a.out_rs = C;
+    a.rows = R;
+    a.cross = cross;
+    a.tw = a.twi = p->tw;
+    a.cin = p->twx;
+    a.ahead = -1;
+    const int rc = launch_rows(&p->kx->k, R, a, st);
+    if (rc) return rc;
+    return mixed_column_groups(p->mxc, p->scratch, C, cross * C, out, G * out_rs, out_rs, C, G, p->mode == kInv,
+                               p->scale, st);
+  }
   a.out = p->scratch;
   a.out_rs = p->rows2d;
   a.rows = p->rows2d;
@@ -1430,6 +1463,27 @@ int fcb_plan_fft2d(long long rows, long long cols, int exponent, float scale, fc
   p->cols2d = cols;
   int rc = plan_common(p, cols, rows, mode);
   if (!rc)
+  {
+    const CrossKernel *kx = cross_kernel(lc, mode == kInv);
+    if (kx && rows / kx->radix <= kCrossMaxRest && rows * cols >= kCrossMinSamples)
+    {
+      p->kx = kx;
+      p->k = &kx->k;
+    }
+  }
+  if (!rc && p->kx)
+  {
+    rc = prepare_kernel(p->k);
+    if (!rc)
+    {
+      cudaFree(p->tw);
+      p->tw = nullptr;
+      rc = build_twiddles(lc, p->k->ept, &p->tw, p->stream);
+    }
+    if (!rc) rc = real_twiddles(rows, rows, &p->twx, p->stream);
+    if (!rc) rc = mixed_create(rows / p->kx->radix, &p->mxc, p->stream);
+  }
+  else if (!rc)
   {
     // 512-thread CTAs hold 4 rows of 4096 (or more of shorter rows), so each
     // transposed store writes whole 32-byte sectors

@@ -366,6 +366,8 @@ struct RowArgs
   long long ahead;      // L2 prefetch distance in tiles (CTAs, or clusters) -- about
                         // half a resident wave, so that tile's rows stream from
                         // HBM into L2 while this tile computes; 0 = off
+  long long cross;      // cross passes: rows between the G rows of a group, a.rows / G;
+                        // cin holds W^k of the column length
   // kR2C reads the twiddle pairs W_2N^2m, W_2N^(2m+1) and then W_2N^(2m+1),
   // W_2N^(2m+2), m < N / 2, from rep; kC2R the twiddles W_2N^k from cin.
   // kChirpconv only (Bluestein rows, whose n samples sit in power-of-two work
@@ -394,7 +396,16 @@ __device__ __forceinline__ void prefetch_l2_bulk(const void *p, uint32_t bytes)
 // kR2C and kC2R are the transforms of real rows of 2N samples, read or written
 // as N complex ones: kR2C splits Z into the N + 1 bins of the half spectrum as
 // it stores, kC2R merges the half spectrum into Z as it loads.
-enum Mode { kFwd = 0, kInv = 1, kFastconv = 2, kChirpconv = 3, kR2C = 4, kC2R = 5 };
+// kFwdCross and kInvCross are the row pass of a 2-D FFT that takes the column
+// transforms' first stage along: the rows of a CTA lie a.cross rows apart (in
+// groups of G, see cross_radix) and are combined by a radix-G step before they
+// are stored, so that the column pass is left with columns of 1 / G the length
+// and can take 64 to 128 bytes of each row at a time.
+enum Mode { kFwd = 0, kInv = 1, kFastconv = 2, kChirpconv = 3, kR2C = 4, kC2R = 5, kFwdCross = 6, kInvCross = 7 };
+
+// Rows that a cross pass combines, of the rows its CTA holds.
+template <class S>
+__host__ __device__ constexpr int cross_radix() { return S::ROWS < 16 ? S::ROWS : 16; }
 
 __device__ __forceinline__ float2 c_mul(float2 a, float2 b)
 {
@@ -475,9 +486,11 @@ __device__ __forceinline__ void row_tile(const RowArgs &a, long long tile, int r
 {
   using S = Sched<LOGN, THREADS, EPTW, ONE_PER_SM>;
   constexpr int RB = S::RB, LRB = S::LRB;
-  constexpr int SIGN = (MODE == kInv || MODE == kC2R) ? +1 : -1;  // direction of the first pass
-  constexpr bool CHIRP = MODE == kChirpconv;
-  constexpr int MD = CHIRP ? kFastconv : MODE == kR2C ? kFwd : MODE == kC2R ? kInv : MODE;  // the transform structure
+  constexpr int SIGN = (MODE == kInv || MODE == kC2R || MODE == kInvCross) ? +1 : -1;  // direction of the first pass
+  constexpr bool CHIRP = MODE == kChirpconv, CROSS = MODE == kFwdCross || MODE == kInvCross;
+  // the transform structure
+  constexpr int MD = CHIRP ? kFastconv : (MODE == kR2C || MODE == kFwdCross) ? kFwd
+                   : (MODE == kC2R || MODE == kInvCross) ? kInv : MODE;
   constexpr int LH1 = ilog2(S::H1);
   constexpr bool CL = S::CS > 1;
   // stage 2 reads its block of D slots from its own CTA only
@@ -489,8 +502,13 @@ __device__ __forceinline__ void row_tile(const RowArgs &a, long long tile, int r
   const int t = threadIdx.x;
   const int rho = CL ? 0 : t / S::TPR;                       // row within CTA
   const int tr = CL ? rank * THREADS + t : t % S::TPR;       // thread within row
-  const long long row = CL ? tile : tile * S::ROWS + rho;
-  const bool active = row < a.rows;
+  // cross pass: row n' + cross * r of the matrix, n' = tile * J + rho % J, r = rho / J
+  constexpr int G = CROSS ? cross_radix<S>() : 1, J = S::ROWS / G;
+  auto row_of = [&](long long tl, int rh) -> long long {
+    return CL ? tl : CROSS ? tl * J + rh % J + a.cross * (rh / J) : tl * S::ROWS + rh;
+  };
+  const long long row = row_of(tile, rho);
+  const bool active = CROSS ? tile * J + rho % J < a.cross : row < a.rows;
 
   // 32-bit base address of every cluster rank's slot array (own array when CS == 1)
   uint32_t peer[S::CS];
@@ -609,7 +627,7 @@ __device__ __forceinline__ void row_tile(const RowArgs &a, long long tile, int r
         {
           const int i = t + THREADS * k;
           const int li = rank * LINES + i;
-          const long long r = row0 + li / LPR;
+          const long long r = CROSS ? row_of(tile + a.ahead, li / LPR) : row0 + li / LPR;
           if (a.ahead > 0 && i < LINES && r < a.rows && (!CHIRP || (li % LPR) * 16 < a.n_in))
             prefetch_l2(a.in + r * a.in_rs + (li % LPR) * 16);
         }
@@ -775,6 +793,37 @@ __device__ __forceinline__ void row_tile(const RowArgs &a, long long tile, int r
     const int tl = t % S::TPRL;
     float2 *dstp = a.out + row * a.out_rs;
     const float2 sc = f2dup(a.scale);
+    if constexpr (CROSS)
+    {
+      // column pair 2m, 2m + 1 of the G rows n' + cross * r: a radix-G step over r,
+      // output q times W^(n' q) (W of the whole column length, a table), to row
+      // cross * q + n'
+      constexpr int LG = ilog2(G);
+#pragma unroll
+      for (int i = 0; i < S::CPT / G; ++i)
+      {
+        const int idx = t + THREADS * i, m = idx % S::HALF, j = idx / S::HALF;
+        const long long np = tile * J + j;
+        cpair z[G];
+#pragma unroll
+        for (int r = 0; r < G; ++r) z[r] = cp_from4(ld_slot<false>(slot_addr((r * J + j) * S::HALF + m)));
+        if (np >= a.cross) continue;
+        DifNet<G, SIGN>::run(z);
+#pragma unroll
+        for (int k = 0; k < G; ++k)
+        {
+          const int q = bitrev(k, LG);
+          if (q != 0)
+          {
+            const float2 w = ldv2(a.cin + np * q);
+            z[k] = SIGN < 0 ? cp_mul<false>(z[k], f2dup(w.x), f2dup(w.y)) : cp_mul<true>(z[k], f2dup(w.x), f2dup(w.y));
+          }
+          reinterpret_cast<float4 *>(a.out + (a.cross * q + np) * a.out_rs)[m] =
+              make_float4(z[k].re.x, z[k].im.x, z[k].re.y, z[k].im.y);
+        }
+      }
+      return;
+    }
     if constexpr (MODE == kR2C)
     {
       // X[k] = E + W_2N^k O, E = (Z[k] + conj Z[N-k]) / 2, O = (Z[k] - conj Z[N-k]) / 2i,

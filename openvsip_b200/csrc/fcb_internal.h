@@ -54,6 +54,15 @@ const KernelInfo *chirp_kernel(int logn, const KernelInfo *like);
 // split of rows that span a cluster: measured 125 us against 89 us for two passes
 // over 256 rows of 65536, each bin pair reading two slots of other CTAs).
 const KernelInfo *real_kernel(int logn, bool inverse, const KernelInfo *like);
+// Row pass of a 2-D transform that combines `radix` rows (fcb_rows_cross.cu):
+// rows of 64 .. 8192 samples.
+struct CrossKernel
+{
+  KernelInfo k;
+  int radix = 1;
+};
+constexpr int kCrossMinLog = 6, kCrossMaxLog = 13;
+const CrossKernel *cross_kernel(int logn, bool inverse);
 int set_variant(int logn, int mode, int threads);
 const KernelInfo *kernel_variant(int logn, int mode, int threads);
 int get_variant(int logn, int mode);
@@ -93,6 +102,11 @@ int mixed_replica(const MixedPlan *p, const float2 *spec, long long spec_rs, lon
 // `count` rows (or, with columns, columns) of a matrix whose rows are in_ld / out_ld apart
 int mixed_transform(MixedPlan *p, bool columns, const float2 *in, long long in_ld, float2 *out, long long out_ld,
                     long long count, bool inverse, float scale, cudaStream_t st);
+// Columns of a stack of `groups` matrices, in_gs / out_gs elements apart, whose rows
+// are in_ld / out_ld apart
+int mixed_column_groups(MixedPlan *p, const float2 *in, long long in_ld, long long in_gs, float2 *out,
+                        long long out_ld, long long out_gs, long long cols, long long groups, bool inverse,
+                        float scale, cudaStream_t st);
 int mixed_conv(MixedPlan *p, const float2 *in, long long in_rs, float2 *out, long long out_rs, long long rows,
                const float2 *rep, long long rep_rs, cudaStream_t st);
 // Bluestein pass over rows of n samples in the plan's work length (>= 2 n - 1)

@@ -71,7 +71,8 @@ struct MrArgs
   long long in_bs, in_es;  // element k of transform r: in[r * in_bs + k * in_es]
   float2 *out;
   long long out_bs, out_es;
-  long long count;         // transforms
+  long long in_gs, out_gs;  // columns: distance of the matrices of a stack (blockIdx.y)
+  long long count;         // transforms (of one matrix)
   int n, ns, C, logC;      // length, stages, transforms per CTA (columns: a power of two)
   MrStage st[kMrStages];
   const float2 *tw;
@@ -313,7 +314,7 @@ __global__ void __launch_bounds__(MAXT, MINB) mixed_kernel(const __grid_constant
   };
   auto load_global = [&](const MrStage &s, int c, int b, auto rc, float2 *x) {
     constexpr int R = decltype(rc)::value;
-    const float2 *p = a.in + (r0 + c) * a.in_bs + b * a.in_es;
+    const float2 *p = a.in + (COL ? blockIdx.y * a.in_gs : 0) + (r0 + c) * a.in_bs + b * a.in_es;
     const long long step = s.S * a.in_es;
     if constexpr (KIND == kMrChirp)
     {
@@ -371,7 +372,7 @@ __global__ void __launch_bounds__(MAXT, MINB) mixed_kernel(const __grid_constant
         Dft<R>::run(x);
         if constexpr (KIND == kMrTransform)
         {
-          float2 *p = a.out + (r0 + c) * a.out_bs;
+          float2 *p = a.out + (COL ? blockIdx.y * a.out_gs : 0) + (r0 + c) * a.out_bs;
 #pragma unroll
           for (int q = 0; q < R; ++q)
             p[q * a.out_es] = swap_if(make_float2(x[q].x * a.scale, x[q].y * a.scale), inv);
@@ -447,7 +448,7 @@ __global__ void __launch_bounds__(MAXT, MINB) mixed_kernel(const __grid_constant
         Dft<R>::run(x);
         if constexpr (KIND == kMrTransform)
         {
-          float2 *p = a.out + (r0 + c) * a.out_bs + b * a.out_es;
+          float2 *p = a.out + (COL ? blockIdx.y * a.out_gs : 0) + (r0 + c) * a.out_bs + b * a.out_es;
           const long long step = s.nb * a.out_es;
 #pragma unroll
           for (int q = 0; q < R; ++q)
@@ -608,20 +609,20 @@ MrConfig configure_rows(const MixedPlan &p, long long count, int sms)
 
 // Columns: C adjacent ones per CTA, so that accesses cover 8 C bytes side by side.  At least 4 (a 32-byte sector)
 // where they fit, more while two CTAs fit an SM and every SM has one.
-MrConfig configure_cols(const MixedPlan &p, long long count, int sms)
+MrConfig configure_cols(const MixedPlan &p, long long count, long long groups, int sms)
 {
   int C = 1;
   while (C < 32 && C < count)
   {
     const long long smem = 16LL * C * p.n;
     if (smem > kMrSmem) break;
-    if (C >= 4 && (smem > kMrSmem / 2 || (count + 2 * C - 1) / (2 * C) < sms)) break;
+    if (C >= 4 && (smem > kMrSmem / 2 || (count + 2 * C - 1) / (2 * C) * groups < sms)) break;
     C *= 2;
   }
   // enough threads for one butterfly each, at most 256 where several CTAs share an SM
   int most = 0;
   for (int k = 0; k < p.ns; ++k) most = std::max(most, p.st[k].nb * C);
-  const int cap = 8LL * C * p.n > kMrSmem / 2 || (count + C - 1) / C <= sms ? 512 : 256;
+  const int cap = 8LL * C * p.n > kMrSmem / 2 || (count + C - 1) / C * groups <= sms ? 512 : 256;
   return {C, std::max(64, std::min(cap, (most + 31) / 32 * 32))};
 }
 
@@ -636,17 +637,17 @@ const void *mixed_fn(int kind, bool col, bool big)
   }
 }
 
-int mixed_launch(MixedPlan *p, int kind, bool col, MrArgs &a, cudaStream_t st)
+int mixed_launch(MixedPlan *p, int kind, bool col, MrArgs &a, cudaStream_t st, long long groups = 1)
 {
   if (a.count <= 0) return FCB_OK;
   MrConfig c;
   const unsigned long long seen = p->last[col].load(std::memory_order_relaxed);
-  if ((long long)(seen >> 24) == a.count)
+  if (groups == 1 && (long long)(seen >> 24) == a.count)
     c = {(int)(seen >> 12 & 0xfff), (int)(seen & 0xfff)};
   else
   {
-    c = col ? configure_cols(*p, a.count, p->sms) : configure_rows(*p, a.count, p->sms);
-    if (a.count < 1LL << 40)
+    c = col ? configure_cols(*p, a.count, groups, p->sms) : configure_rows(*p, a.count, p->sms);
+    if (a.count < 1LL << 40 && groups == 1)
       p->last[col].store((unsigned long long)a.count << 24 | (unsigned)c.C << 12 | (unsigned)c.threads,
                          std::memory_order_relaxed);
   }
@@ -659,11 +660,11 @@ int mixed_launch(MixedPlan *p, int kind, bool col, MrArgs &a, cudaStream_t st)
   a.tw = p->tw;
   a.rev = p->rev;
   const long long grid = (a.count + c.C - 1) / c.C;
-  if (grid > 0x7fffffffLL) return set_error(FCB_ERR_INVALID, "too many rows in one call");
+  if (grid > 0x7fffffffLL || groups > 65535) return set_error(FCB_ERR_INVALID, "too many rows in one call");
   const size_t smem = p->ns > 1 ? sizeof(float2) * (size_t)c.C * p->n : 0;
   const void *fn = mixed_fn(kind, col, c.threads > 256);
   void *params[] = {&a};
-  const cudaError_t e = cudaLaunchKernel(fn, dim3((unsigned)grid), dim3(c.threads), params, smem, st);
+  const cudaError_t e = cudaLaunchKernel(fn, dim3((unsigned)grid, (unsigned)groups), dim3(c.threads), params, smem, st);
   return e == cudaSuccess ? FCB_OK : cuda_error(e, "mixed-radix kernel launch");
 }
 
@@ -793,6 +794,24 @@ int mixed_transform(MixedPlan *p, bool columns, const float2 *in, long long in_l
   a.inverse = inverse;
   a.scale = scale;
   return mixed_launch(p, kMrTransform, columns, a, st);
+}
+
+int mixed_column_groups(MixedPlan *p, const float2 *in, long long in_ld, long long in_gs, float2 *out,
+                        long long out_ld, long long out_gs, long long cols, long long groups, bool inverse,
+                        float scale, cudaStream_t st)
+{
+  MrArgs a = {};
+  a.in = in;
+  a.out = out;
+  a.in_bs = a.out_bs = 1;
+  a.in_es = in_ld;
+  a.out_es = out_ld;
+  a.in_gs = in_gs;
+  a.out_gs = out_gs;
+  a.count = cols;
+  a.inverse = inverse;
+  a.scale = scale;
+  return mixed_launch(p, kMrTransform, true, a, st, groups);
 }
 
 int mixed_conv(MixedPlan *p, const float2 *in, long long in_rs, float2 *out, long long out_rs, long long rows,

@@ -6,6 +6,8 @@
 #include "fcb_engine.cuh"
 #include "fcb_internal.h"
 
+#include <mutex>
+
 namespace fcb {
 
 template <int LOGN, int MODE, int T, int EPTW = 32>

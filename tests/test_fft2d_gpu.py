@@ -64,3 +64,25 @@ def test_fft2d_rejects_unsupported_sizes():
     for rows, cols in ((0, 8), (8, 40000), (70000, 4)):
         with pytest.raises(FcbError):
             Fft2d(rows, cols, fft_fwd)
+
+
+# the row pass with the columns' first stage: radix 16 (several groups a CTA), 8, 4 and 2, the
+# longest rest of the columns
+@pytest.mark.parametrize("rows,cols", [(16384, 128), (2048, 1024), (1024, 2048), (512, 4096), (8192, 512), (256, 8192),
+                                       (8192, 8192)])
+def test_fft2d_cross_pass_vs_fp64(oracle, rows, cols):
+    import torch
+    rng = np.random.default_rng(rows + cols)
+    x = crandn(rng, (rows, cols))
+    f = Fft2d(rows, cols, fft_fwd, 0.5)
+    want = 0.5 * np.fft.fft2(x.astype(np.complex128))
+    out = torch.zeros(rows, cols + 5, dtype=torch.complex64, device="cuda")
+    dx = torch.from_numpy(x).cuda()
+    f(dx, out[:, 1:cols + 1])  # unaligned rows
+    got = out[:, 1:cols + 1].cpu().numpy()
+    assert oracle.rel_l2(got, want) <= RTOL
+    assert not out[:, :1].any() and not out[:, cols + 1:].any()
+    f(dx, dx)  # in place
+    assert np.array_equal(dx.cpu().numpy(), got)
+    g = Fft2d(rows, cols, fft_inv, 2.0 / (rows * cols))
+    assert oracle.rel_l2(g(dx).cpu().numpy(), x) <= RTOL
