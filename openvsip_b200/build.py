@@ -22,11 +22,9 @@ FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler", 
          f"-I{os.path.join(ROOT, 'include')}", f"-I{CSRC}"]
 
 SOURCES = ["fcb_rows_conv.cu", "fcb_rows_fwd.cu", "fcb_rows_inv.cu", "fcb_rows_r2c.cu",
-           "fcb_rows_c2r.cu", "fcb_rows_cross.cu", "fcb_batch.cu", "fcb_mixed.cu", "fcb200.cu",
+           "fcb_rows_c2r.cu", "fcb_rows_cross.cu", "fcb_batch.cu", "fcb_mixed_conv.cu", "fcb_mixed_rows.cu",
+           "fcb_mixed_cols.cu", "fcb_mixed.cu", "fcb200.cu",
            "fcb_api.cu", "fcb_bluestein.cu", "fcb_real.cu", "fcb_hostcopy.cu"]
-
-# The mixed-radix kernels dominate the build when compiled one after another.
-EXTRA = {"fcb_mixed.cu": ["--split-compile=0"]}
 
 
 def nvcc() -> str:
@@ -60,7 +58,7 @@ def build(verbose: bool = False, force: bool = False) -> str:
         obj = os.path.join(BUILD, s.replace(".cu", ".o"))
         objs.append(obj)
         if force or _stale(obj, [src] + headers):
-            cmd = [nvcc(), *ARCH, *FLAGS, *EXTRA.get(s, []), "-c", src, "-o", obj]
+            cmd = [nvcc(), *ARCH, *FLAGS, "-c", src, "-o", obj]
             jobs.append(cmd)
 
     def run(cmd):

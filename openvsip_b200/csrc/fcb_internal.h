@@ -109,11 +109,6 @@ int mixed_column_groups(MixedPlan *p, const float2 *in, long long in_ld, long lo
                         float scale, cudaStream_t st);
 int mixed_conv(MixedPlan *p, const float2 *in, long long in_rs, float2 *out, long long out_rs, long long rows,
                const float2 *rep, long long rep_rs, cudaStream_t st);
-// Bluestein pass over rows of n samples in the plan's work length (>= 2 n - 1)
-int mixed_chirp(MixedPlan *p, const float2 *in, long long in_rs, float2 *out, long long out_rs, long long rows,
-                long long n, const float2 *cin, long long cin_rs, const float2 *cout, const float2 *rep,
-                cudaStream_t st);
-
 // Real-input row FFTs (fcb_real.cu).
 int real_twiddles(long long n, long long count, float2 **out, cudaStream_t st);
 int real_twiddle_pairs(long long n, float4 **out, cudaStream_t st);
