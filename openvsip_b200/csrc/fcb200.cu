@@ -192,6 +192,7 @@ __global__ void dft_fp64_kernel(const float2 *in, const double2 *w, unsigned n, 
 __global__ void vmmul_kernel(const float2 *v, const float2 *m, long long m_rs, float2 *out,
                              long long out_rs, long long rows, long long cols)
 {
+  begin_after_previous();
   long long total = rows * cols;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
        i += (long long)gridDim.x * blockDim.x)
@@ -354,27 +355,44 @@ int launch_rows(const KernelInfo *k, long long rows, const RowArgs &args, cudaSt
   if (rows <= 0) return FCB_OK;
   long long ctas = k->cluster > 1 ? rows * k->cluster : (rows + k->rows_per_cta - 1) / k->rows_per_cta;
   if (ctas > 0x7fffffffLL) return set_error(FCB_ERR_INVALID, "too many rows in one call");
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)ctas);
-  cfg.blockDim = dim3(k->threads);
-  cfg.dynamicSmemBytes = k->smem;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  if (k->cluster > 1)
-  {
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = k->cluster;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-  }
   RowArgs a = args;
   if (a.ahead < 0) a.ahead = (k->resident_tiles + 1) / 2;  // half a resident wave ahead (measured best)
   void *params[] = {&a};
-  cudaError_t e = cudaLaunchKernelExC(&cfg, k->fn, params);
-  if (e != cudaSuccess) return cuda_error(e, "row kernel launch");
-  return FCB_OK;
+  return launch_kernel(k->fn, dim3((unsigned)ctas), k->threads, k->cluster, k->smem, params, st, "row kernel launch");
+}
+
+int launch_kernel(const void *fn, dim3 grid, int threads, int cluster, size_t smem, void **params, cudaStream_t st,
+                  const char *what)
+{
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  cfg.attrs = attr;
+  cfg.numAttrs = 0;
+  if (cluster > 1)
+  {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+    attr[cfg.numAttrs].val.clusterDim.x = cluster;
+    attr[cfg.numAttrs].val.clusterDim.y = 1;
+    attr[cfg.numAttrs].val.clusterDim.z = 1;
+    ++cfg.numAttrs;
+  }
+  // a captured launch stays an ordinary graph node: programmatic edges would not
+  // survive every caller's capture queries
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone)
+  {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[cfg.numAttrs].val.programmaticStreamSerializationAllowed = 1;
+    ++cfg.numAttrs;
+  }
+  else
+    cudaGetLastError();
+  const cudaError_t e = cudaLaunchKernelExC(&cfg, fn, params);
+  return e == cudaSuccess ? FCB_OK : cuda_error(e, what);
 }
 
 int build_twiddles(int logn, int ept, float4 **out, cudaStream_t st)
@@ -434,10 +452,8 @@ int launch_vmmul(const float2 *v, const float2 *m, long long m_rs, float2 *out, 
   if (total <= 0) return FCB_OK;
   long long blocks = (total + 255) / 256;
   if (blocks > 148 * 64) blocks = 148 * 64;
-  vmmul_kernel<<<(unsigned)blocks, 256, 0, st>>>(v, m, m_rs, out, out_rs, rows, cols);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return cuda_error(e, "vmmul launch");
-  return FCB_OK;
+  void *params[] = {&v, &m, &m_rs, &out, &out_rs, &rows, &cols};
+  return launch_kernel((const void *)&vmmul_kernel, dim3((unsigned)blocks), 256, 1, 0, params, st, "vmmul launch");
 }
 
 int launch_transpose(const float2 *in, long long in_rs, float2 *out, long long out_rs, long long rows,

@@ -1070,11 +1070,24 @@ __device__ __forceinline__ void row_tile(const RowArgs &a, long long tile, int r
   }
 }
 
+// Every kernel of the library that a call launches begins with these two, and is
+// launched with the programmatic-serialization attribute (see launch_kernel), so
+// that the launch of a call overlaps the end of the one before it: wait until the
+// work queued before this kernel is complete and visible, then let the next
+// kernel's CTAs take free places (they wait in turn).  Nothing may touch global
+// memory before the wait.
+__device__ __forceinline__ void begin_after_previous()
+{
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // Standalone launch: one tile per CTA, or per cluster of CS CTAs.
 template <int LOGN, int MODE, int THREADS, int EPTW = 32>
 __global__ void __launch_bounds__(THREADS, (Sched<LOGN, THREADS, EPTW>::MINB)) rows_kernel(RowArgs a)
 {
   using S = Sched<LOGN, THREADS, EPTW>;
+  begin_after_previous();
   if constexpr (S::CS > 1)
     row_tile<LOGN, MODE, THREADS, EPTW>(a, blockIdx.x / S::CS, (int)cg::this_cluster().block_rank(), 0, true);
   else

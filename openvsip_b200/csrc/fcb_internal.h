@@ -67,6 +67,10 @@ int set_variant(int logn, int mode, int threads);
 const KernelInfo *kernel_variant(int logn, int mode, int threads);
 int get_variant(int logn, int mode);
 int prepare_kernel(const KernelInfo *k);
+// Launches a kernel that starts with begin_after_previous(), in clusters of `cluster`
+// CTAs, so that its launch overlaps the end of the kernel before it in the stream.
+int launch_kernel(const void *fn, dim3 grid, int threads, int cluster, size_t smem, void **params, cudaStream_t st,
+                  const char *what);
 int launch_rows(const KernelInfo *k, long long rows, const RowArgs &args, cudaStream_t st);
 
 int build_twiddles(int logn, int ept, float4 **out, cudaStream_t st);

@@ -177,8 +177,8 @@ int mixed_launch(MixedPlan *p, int kind, bool col, MrArgs &a, cudaStream_t st, l
   const size_t smem = p->ns > 1 ? sizeof(float2) * (size_t)c.C * p->n : 0;
   const void *fn = mixed_fn(kind, col, c.threads > 256);
   void *params[] = {&a};
-  const cudaError_t e = cudaLaunchKernel(fn, dim3((unsigned)grid, (unsigned)groups), dim3(c.threads), params, smem, st);
-  return e == cudaSuccess ? FCB_OK : cuda_error(e, "mixed-radix kernel launch");
+  return launch_kernel(fn, dim3((unsigned)grid, (unsigned)groups), c.threads, 1, smem, params, st,
+                       "mixed-radix kernel launch");
 }
 
 }  // namespace

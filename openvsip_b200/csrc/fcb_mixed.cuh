@@ -39,6 +39,8 @@
 // 1.13.
 #pragma once
 
+#include "fcb_engine.cuh"
+
 #include <cuda_runtime.h>
 
 #include <type_traits>
@@ -281,6 +283,7 @@ template <int KIND, bool COL, int MAXT, int MINB>
 __global__ void __launch_bounds__(MAXT, MINB) mixed_kernel(const __grid_constant__ MrArgs a)
 {
   extern __shared__ float2 sm[];
+  begin_after_previous();
   const int t = threadIdx.x, T = blockDim.x;
   const long long r0 = (long long)blockIdx.x * a.C;
   const int cnt = (int)min((long long)a.C, a.count - r0);  // transforms of this CTA
