@@ -79,5 +79,28 @@ def build(verbose: bool = False, force: bool = False) -> str:
     return LIB
 
 
+def build_torch(force: bool = False) -> str:
+    """The native host path for CUDA tensors (csrc/fcb_torch.cpp), a Python
+    extension module against the installed torch."""
+    import sysconfig
+
+    import torch
+    src = os.path.join(CSRC, "fcb_torch.cpp")
+    out = os.path.join(HERE, "_fcb_torch.so")
+    if not force and not _stale(out, [src]):
+        return out
+    tdir = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(os.path.realpath(nvcc())))
+    cmd = [shutil.which("g++") or "g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           f"-I{sysconfig.get_paths()['include']}", f"-I{tdir}/include", f"-I{tdir}/include/torch/csrc/api/include",
+           f"-I{cuda}/include", src, "-o", out, f"-L{tdir}/lib", "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"g++ failed: {' '.join(cmd)}\n{r.stdout}\n{r.stderr}")
+    return out
+
+
 if __name__ == "__main__":
     print(build(verbose="-v" in sys.argv, force="-f" in sys.argv))
+    print(build_torch(force="-f" in sys.argv))

@@ -141,13 +141,15 @@ int check_device()
   if (e != cudaSuccess || count == 0) return set_error(FCB_ERR_NODEVICE, "no CUDA device: %s", cudaGetErrorString(e));
   int dev = 0;
   cudaGetDevice(&dev);
-  cudaDeviceProp p;
-  e = cudaGetDeviceProperties(&p, dev);
-  if (e != cudaSuccess) return cuda_error(e, "cudaGetDeviceProperties");
+  // two attributes: cudaGetDeviceProperties took 2.5 ms, nine tenths of making a plan
+  int major = 0, minor = 0;
+  e = cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&minor, cudaDevAttrComputeCapabilityMinor, dev);
+  if (e != cudaSuccess) return cuda_error(e, "cudaDeviceGetAttribute");
   // sm_100a code runs on compute capability 10.0 only
-  if (p.major != 10 || p.minor != 0)
+  if (major != 10 || minor != 0)
     return set_error(FCB_ERR_NODEVICE, "device %d is sm_%d%d; this library is built for sm_100a (compute capability 10.0)",
-                     dev, p.major, p.minor);
+                     dev, major, minor);
   return FCB_OK;
 }
 

@@ -142,6 +142,34 @@ def _put_transposed(out, yt):
     return out
 
 
+def _load_native(*args):
+    """Stands for the native call path (csrc/fcb_torch.cpp) until the first call
+    on a tensor: loads it and makes that call.  Without the module every call
+    takes the ctypes path."""
+    global _native
+    import sys
+    if "torch" not in sys.modules:
+        return None
+    try:
+        from . import _fcb_torch
+    except ImportError:
+        _native = _no_native
+    else:
+        L = lib()
+        _fcb_torch.bind(*(ctypes.cast(f, ctypes.c_void_p).value for f in (
+            L.fcb_set_stream, L.fcb_exec, L.fcb_exec_r2c, L.fcb_exec_c2r, L.fcb_exec_cols)))
+        _native = _fcb_torch.exec
+    return _native(*args)
+
+
+def _no_native(*args):
+    return None
+
+
+_native = _load_native  # (kind, plan, in, out, n_in, n_out) -> status, or None: not plain CUDA matrices
+_ROWS, _R2C, _C2R, _COLS = range(4)
+
+
 def _plain_matrix(x, writable: bool):
     """(pointer, rows, cols, row stride, where) of a complex64 matrix with
     unit-stride rows that its memory holds as they are (no lazy conjugate, no
@@ -172,16 +200,18 @@ def _same_or_apart(a, b) -> bool:
 
 class _Plan:
     _handle = None
-    _stream = None  # the stream handle last bound to the plan (fcb_set_stream)
 
     def _bind_stream(self, where) -> None:
-        """Device calls run on the current torch stream; the plan is told only
-        when that stream changes."""
+        """Device calls run on the current torch stream."""
         if where == _lib.FCB_DEVICE:
-            s = _stream_handle()
-            if s != self._stream:
-                check(lib().fcb_set_stream(self._handle, ctypes.c_void_p(s)))
-                self._stream = s
+            check(lib().fcb_set_stream(self._handle, ctypes.c_void_p(_stream_handle())))
+
+    def _device_call(self, kind, inp, out, n_in, n_out) -> bool:
+        """The whole call natively, for plain CUDA matrices; False for others."""
+        rc = _native(kind, self._handle.value, inp, out, n_in, n_out)
+        if rc:
+            check(rc)
+        return rc is not None
 
     def __del__(self):
         h, self._handle = self._handle, None
@@ -203,11 +233,13 @@ class _Plan:
                 "threads": th.value}
 
     def _exec(self, inp, out, wait: bool = True):
+        if type(inp) is not np.ndarray and self._device_call(_ROWS, inp, out, self._n, self._n):
+            return out
         ip, r, c, irs, iw = _desc(inp, False)
         op, r2, c2, ors, ow = _desc(out, True)
         if (r, c) != (r2, c2):
             raise ValueError(f"shape mismatch {(r, c)} vs {(r2, c2)}")
-        n = getattr(self, "_n", self.cols)  # transform length (Fftm along columns: rows)
+        n = self._n  # transform length (Fftm along columns: rows)
         if c != n:
             raise ValueError(f"row length {c} != planned {n}")
         if iw != ow:
@@ -275,6 +307,8 @@ class Fftm(_Plan):
         return self._exec(inout, inout)
 
     def _columns(self, inp, out):
+        if self._col_kernel and type(inp) is not np.ndarray and self._device_call(_COLS, inp, out, self._n, self.cols):
+            return out
         a = _plain_matrix(inp, False) if self._col_kernel else None
         b = _plain_matrix(out, True) if a else None
         if not (a and b and a[1:3] == b[1:3] and a[1] == self._n and a[2] <= self.cols and a[4] == b[4]
@@ -332,6 +366,9 @@ class FftmReal(_Plan):
 
     def _rows(self, inp, out):
         fwd = self.exponent == _lib.FCB_FORWARD
+        if type(inp) is not np.ndarray and self._device_call(
+                _R2C if fwd else _C2R, inp, out, self.n if fwd else self.bins, self.bins if fwd else self.n):
+            return out
         ip, r, c, irs, iw = _desc(inp, False, real=fwd)
         op, r2, c2, ors, ow = _desc(out, True, real=not fwd)
         want_in, want_out = (self.n, self.bins) if fwd else (self.bins, self.n)
@@ -359,6 +396,7 @@ class Fft2d(_Plan):
         h = ctypes.c_void_p()
         check(lib().fcb_plan_fft2d(self.rows, self.cols, self.exponent, self.scale, ctypes.byref(h)))
         self._handle = h
+        self._n = self.cols
 
     def __call__(self, inp, out=None):
         if out is None:
@@ -384,6 +422,7 @@ class Fastconv(_Plan):
             weights = np.ascontiguousarray(weights, dtype=np.complex64)
         wp, wr, wc, wrs, ww = _desc(weights, False)
         self.rows, self.cols = int(rows), int(wc)
+        self._n = self.cols
         self.replica_rows = wr
         h = ctypes.c_void_p()
         check(lib().fcb_plan_fastconv(self.cols, self.rows, ctypes.c_void_p(wp), wr, wrs,
