@@ -7,7 +7,9 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdarg>
+#include <cstdint>
 #include <cstdio>
 #include <cstring>
 #include <mutex>
@@ -189,17 +191,42 @@ __global__ void dft_fp64_kernel(const float2 *in, const double2 *w, unsigned n, 
   }
 }
 
-__global__ void vmmul_kernel(const float2 *v, const float2 *m, long long m_rs, float2 *out,
-                             long long out_rs, long long rows, long long cols)
+// out[r][c] = v[c] m[r][c].  A thread keeps its columns' multipliers in registers and
+// goes down the rows, so an element costs its own load and store and nothing else
+// (HBM-bound: 16 bytes a sample; with a grid-stride loop over elements and its 64-bit
+// division, 1024 x 8192 took 32.8 us against 19.5, 4096 x 1000 18.4 against 7.0).  VEC: two columns a thread in 16-byte accesses,
+// for rows that all start 16-byte aligned.
+template <bool VEC>
+__global__ void __launch_bounds__(256) vmmul_kernel(const float2 *v, const float2 *m, long long m_rs, float2 *out,
+                                                    long long out_rs, long long rows, long long cols)
 {
   begin_after_previous();
-  long long total = rows * cols;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
-       i += (long long)gridDim.x * blockDim.x)
+  const long long c = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * (VEC ? 2 : 1);
+  if (c >= cols) return;
+  const long long step = gridDim.y;
+  using V = std::conditional_t<VEC, float4, float2>;
+  const float2 w0 = v[c], w1 = VEC ? v[c + 1] : w0;
+  constexpr int B = 4;  // rows in flight (loads first: out may be m, so the compiler keeps the order)
+  for (long long r = blockIdx.y; r < rows; r += B * step)
   {
-    long long r = i / cols, c = i % cols;
-    float2 a = v[c], b = m[r * m_rs + c];
-    out[r * out_rs + c] = make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+    V b[B];
+#pragma unroll
+    for (int k = 0; k < B; ++k)
+      if (r + k * step < rows) b[k] = *reinterpret_cast<const V *>(m + (r + k * step) * m_rs + c);
+#pragma unroll
+    for (int k = 0; k < B; ++k)
+    {
+      if (r + k * step >= rows) break;
+      V o;
+      o.x = w0.x * b[k].x - w0.y * b[k].y;
+      o.y = w0.x * b[k].y + w0.y * b[k].x;
+      if constexpr (VEC)
+      {
+        o.z = w1.x * b[k].z - w1.y * b[k].w;
+        o.w = w1.x * b[k].w + w1.y * b[k].z;
+      }
+      *reinterpret_cast<V *>(out + (r + k * step) * out_rs + c) = o;
+    }
   }
 }
 
@@ -448,12 +475,17 @@ int replica_spectrum_dev(const float2 *rep_dev, long long n, int matched, float2
 int launch_vmmul(const float2 *v, const float2 *m, long long m_rs, float2 *out, long long out_rs,
                  long long rows, long long cols, cudaStream_t st)
 {
-  long long total = rows * cols;
-  if (total <= 0) return FCB_OK;
-  long long blocks = (total + 255) / 256;
-  if (blocks > 148 * 64) blocks = 148 * 64;
+  if (rows <= 0 || cols <= 0) return FCB_OK;
+  auto even = [](const float2 *p, long long rs) { return reinterpret_cast<uintptr_t>(p) % 16 == 0 && rs % 2 == 0; };
+  const bool vec = cols % 2 == 0 && even(m, m_rs) && even(out, out_rs);
+  const long long gx = (cols / (vec ? 2 : 1) + 255) / 256;
+  if (gx > 0x7fffffffLL) return set_error(FCB_ERR_INVALID, "too many columns in one call");
+  // eight CTAs for every SM, at most sixteen rows a thread
+  const long long gy = std::min<long long>(65535, std::max<long long>(std::min<long long>(rows, (148 * 8 + gx - 1) / gx),
+                                                                      rows / 16));
   void *params[] = {&v, &m, &m_rs, &out, &out_rs, &rows, &cols};
-  return launch_kernel((const void *)&vmmul_kernel, dim3((unsigned)blocks), 256, 1, 0, params, st, "vmmul launch");
+  return launch_kernel(vec ? (const void *)&vmmul_kernel<true> : (const void *)&vmmul_kernel<false>,
+                       dim3((unsigned)gx, (unsigned)gy), 256, 1, 0, params, st, "vmmul launch");
 }
 
 int launch_transpose(const float2 *in, long long in_rs, float2 *out, long long out_rs, long long rows,
