@@ -367,19 +367,46 @@ int prepare_kernel(const KernelInfo *k)
   // Idempotent; cheap after the first call per device.
   cudaError_t e = cudaFuncSetAttribute(k->fn, cudaFuncAttributeMaxDynamicSharedMemorySize, k->smem);
   if (e != cudaSuccess) return cuda_error(e, "cudaFuncSetAttribute(smem)");
-  // tiles resident at once: the L2 prefetch distance
+  // tiles resident at once: the L2 prefetch distance, and the bound of a call of few rows
   int dev = 0, sms = 0, per_sm = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k->fn, k->threads, k->smem);
   if (e != cudaSuccess) return cuda_error(e, "occupancy query");
   const_cast<KernelInfo *>(k)->resident_tiles = (long long)sms * (per_sm > 0 ? per_sm : 1) / k->cluster;
+  if (!k->few) return FCB_OK;
+  const int rc = prepare_kernel(k->few);
+  if (rc || k->few->cluster == 1) return rc;
+  // clusters lie within a GPC: fewer fit than the SM count says
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(sms / k->few->cluster * k->few->cluster));
+  cfg.blockDim = dim3(k->few->threads);
+  cfg.dynamicSmemBytes = k->few->smem;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = k->few->cluster;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  int clusters = 0;
+  e = cudaOccupancyMaxActiveClusters(&clusters, k->few->fn, &cfg);
+  if (e != cudaSuccess) return cuda_error(e, "cluster occupancy query");
+  // one CTA an SM: with two, the ordinary kernel's row is as short
+  k->few->resident_tiles = std::min(clusters, sms / k->few->cluster);
   return FCB_OK;
 }
 
 int launch_rows(const KernelInfo *k, long long rows, const RowArgs &args, cudaStream_t st)
 {
   if (rows <= 0) return FCB_OK;
+  // Few rows: the kernel with the shortest row where all of them are resident at once
+  // (that is one or two CTAs an SM; beyond, the ordinary kernel's four CTAs an SM
+  // measured as fast or faster).  Fast convolution, 64 rows of 512 / 2048 / 4096 /
+  // 8192 samples: 4.4 / 5.5 / 5.7 / 8.5 -> 3.4 / 4.2 / 4.6 / 7.2 us; 512 rows of 4096 11.5 /
+  // 11.7, 8192 of 2048 65.8 / 70.3.
+  // (A transposing pass needs whole rows in a CTA, which the long rows' form splits.)
+  if (k->few && !args.transpose_out && (rows + k->few->rows_per_cta - 1) / k->few->rows_per_cta <= k->few->resident_tiles) k = k->few;
   long long ctas = k->cluster > 1 ? rows * k->cluster : (rows + k->rows_per_cta - 1) / k->rows_per_cta;
   if (ctas > 0x7fffffffLL) return set_error(FCB_ERR_INVALID, "too many rows in one call");
   RowArgs a = args;

@@ -16,6 +16,7 @@
 #include "fcb200.h"
 #include "fcb_engine.cuh"
 #include "fcb_internal.h"
+#include "fcb_rows.cuh"
 
 #include <cuda_runtime.h>
 
@@ -100,30 +101,15 @@ int scale_copy(const float2 *in, float2 *out, long long total, float s, cudaStre
 // Kernel table of the kChirpconv mode: work rows of 8 .. 65536 samples, the
 // same variants as the other modes ([0] 256, [1] 512, [2] 128 threads with 32
 // samples each, [3] 256 threads with 64 samples for 16384-sample rows).
-template <int LOGN, int T, int EPTW = 32>
-static KernelInfo chirp_info()
-{
-  using S = Sched<LOGN, T, EPTW>;
-  KernelInfo k;
-  k.fn = (const void *)&rows_kernel<LOGN, kChirpconv, T, EPTW>;
-  k.threads = T;
-  k.cluster = S::CS;
-  k.rows_per_cta = S::ROWS;
-  k.smem = S::SMEM;
-  k.tw_bytes = S::tw_bytes();
-  k.ept = EPTW;
-  return k;
-}
-
 template <int LOGN>
 static void fill_chirp(KernelInfo (*tab)[kVariants])
 {
   if constexpr (LOGN >= 3)
   {
-    tab[LOGN][0] = chirp_info<LOGN, 256>();
-    if constexpr (LOGN >= kMin512) tab[LOGN][1] = chirp_info<LOGN, 512>();
-    if constexpr (LOGN >= kMin128 && LOGN <= kMax128) tab[LOGN][2] = chirp_info<LOGN, 128>();
-    if constexpr (LOGN >= kWideLog && LOGN <= kWideMaxLog) tab[LOGN][3] = chirp_info<LOGN, 256, 64>();
+    tab[LOGN][0] = rows_info<LOGN, kChirpconv, 256>();
+    if constexpr (LOGN >= kMin512) tab[LOGN][1] = rows_info<LOGN, kChirpconv, 512>();
+    if constexpr (LOGN >= kMin128 && LOGN <= kMax128) tab[LOGN][2] = rows_info<LOGN, kChirpconv, 128>();
+    if constexpr (LOGN >= kWideLog && LOGN <= kWideMaxLog) tab[LOGN][3] = rows_info<LOGN, kChirpconv, 256, 64>();
     fill_chirp<LOGN - 1>(tab);
   }
 }

@@ -481,7 +481,13 @@ __device__ __forceinline__ void half_wait()
 // while consecutive tiles have the same length).  The caller guarantees that
 // no thread of the CTA (or of the CS CTAs) still reads the slot array of a
 // previous tile.
-template <int LOGN, int MODE, int THREADS, int EPTW = 32, int ONE_PER_SM = 0>
+//
+// FEW: for grids that leave each SM one or two CTAs, where a row's own latency is
+// what the call takes.  The kernel may use all registers, so its replica loads are
+// issued at once before the last stage reads its slots (four at a time they cost
+// a memory latency each batch); nothing is prefetched for later tiles.  The
+// arithmetic is the same.
+template <int LOGN, int MODE, int THREADS, int EPTW = 32, int ONE_PER_SM = 0, bool FEW = false>
 __device__ __forceinline__ void row_tile(const RowArgs &a, long long tile, int rank, int rank_base, bool copy_tw)
 {
   using S = Sched<LOGN, THREADS, EPTW, ONE_PER_SM>;
@@ -537,6 +543,16 @@ __device__ __forceinline__ void row_tile(const RowArgs &a, long long tile, int r
                    :: "r"(tw_base + 16u * i), "l"(src + i) : "memory");
     asm volatile("cp.async.commit_group;" ::: "memory");
   }
+
+  // The rows of a CTA exchange nothing with each other: in the transforms a barrier
+  // over the threads of a row lets them run out of phase (4096 x 4096 2-D, whose CTAs
+  // hold four rows: 144 -> 141 us; the fused kernels gained nothing by it, and the
+  // wide batch kernel lost 2 %).
+  auto row_sync = [&]() {
+    if constexpr (CL) cluster_sync();
+    else if constexpr (MD == kFastconv) __syncthreads();
+    else group_sync<S::TPR, THREADS>(t);
+  };
 
   cpair c[S::CPT];
 
@@ -610,6 +626,7 @@ __device__ __forceinline__ void row_tile(const RowArgs &a, long long tile, int r
     // bulk prefetch when that part is 16-byte aligned (measured 6 % faster at
     // 65536 samples; at 32768 samples and for single-CTA rows the per-line
     // prefetch measured as fast or faster).
+    if constexpr (!FEW)
     {
       constexpr int LPR = S::N >= 16 ? S::N / 16 : 1;          // 128-byte lines per row
       constexpr int LINES = S::ROWS * LPR / S::CS;             // lines of this CTA's part
@@ -678,8 +695,14 @@ __device__ __forceinline__ void row_tile(const RowArgs &a, long long tile, int r
   }
   if constexpr (S::NS > 1)
   {
-    if (S::TWS > 0 && copy_tw) asm volatile("cp.async.wait_all;" ::: "memory");
-    if constexpr (CL) cluster_sync(); else __syncthreads();
+    if (S::TWS > 0 && copy_tw)
+    {
+      // the whole CTA reads the twiddles that each thread copied a part of
+      asm volatile("cp.async.wait_all;" ::: "memory");
+      if constexpr (CL) cluster_sync(); else __syncthreads();
+    }
+    else
+      row_sync();
   }
 
   // ---------------- stages 2..NS, direction SIGN ----------------
@@ -700,13 +723,19 @@ __device__ __forceinline__ void row_tile(const RowArgs &a, long long tile, int r
     // arithmetic.
     if constexpr (s == 2 && S::STAGGER)
       if (t >= THREADS / 2) half_wait<15, THREADS>();
+    constexpr int RA = FEW ? RB : 4;  // replica entries loaded together
+    float4 ra[RA];
+    if constexpr (MD == kFastconv && s == S::NS && FEW)
+    {
+#pragma unroll
+      for (int i = 0; i < RB; ++i) ra[i] = ldv4(rp + i * S::TPR + tr);
+    }
 #pragma unroll
     for (int r = 0; r < RB; ++r)
       c[r] = cp_from4(ld_slot<false>(slot_addr(SlotMap<S>::local(base + St * r, rho))));
     if constexpr (s == 2 && S::STAGGER)
       if (t < THREADS / 2) half_arrive<15, THREADS>();
-    float4 ra[4];  // replica entries, four at a time
-    if constexpr (MD == kFastconv && s == S::NS)
+    if constexpr (MD == kFastconv && s == S::NS && !FEW)
     {
 #pragma unroll
       for (int i = 0; i < 4; ++i) ra[i] = ldv4(rp + i * S::TPR + tr);
@@ -735,15 +764,15 @@ __device__ __forceinline__ void row_tile(const RowArgs &a, long long tile, int r
     if constexpr (MD == kFastconv && s == S::NS)
     {
 #pragma unroll
-      for (int b = 0; b < RB; b += 4)
+      for (int b = 0; b < RB; b += RA)
       {
         if (b > 0)
         {
 #pragma unroll
-          for (int i = 0; i < 4; ++i) ra[i] = ldv4(rp + (b + i) * S::TPR + tr);
+          for (int i = 0; i < RA; ++i) ra[i] = ldv4(rp + (b + i) * S::TPR + tr);
         }
 #pragma unroll
-        for (int i = 0; i < 4; ++i) c[b + i] = cp_mul4(c[b + i], ra[i]);
+        for (int i = 0; i < RA; ++i) c[b + i] = cp_mul4(c[b + i], ra[i]);
       }
     }
     if constexpr (s < S::NS)
@@ -781,14 +810,15 @@ __device__ __forceinline__ void row_tile(const RowArgs &a, long long tile, int r
         dst[i] = sigma / S::D + S::H1 * digitrev16(sigma % S::D, S::NS - 1, LRB);
       }
     }
-    if constexpr (CL) cluster_sync(); else __syncthreads();
+    row_sync();
 #pragma unroll
     for (int i = 0; i < S::CPT; ++i)
     {
       const int m = dst[i];
       st_slot<CL>(peer[SlotMap<S>::owner(m)] + 16u * swz_(SlotMap<S>::local(m, rho)), cp_to4(c[i]));
     }
-    if constexpr (CL) cluster_sync(); else __syncthreads();
+    // the transposing and the cross pass read other rows of the CTA
+    if (!CL && (CROSS || a.transpose_out)) __syncthreads(); else row_sync();
     // natural-order read of this CTA's part of the row, scale, store.
     const int tl = t % S::TPRL;
     float2 *dstp = a.out + row * a.out_rs;
@@ -991,7 +1021,7 @@ __device__ __forceinline__ void row_tile(const RowArgs &a, long long tile, int r
     {
 #pragma unroll
       for (int qp = 0; qp < S::H1; ++qp) tw1[qp] = ldv4(a.twi + qp * S::D + tr);
-      if constexpr (CL) cluster_sync(); else __syncthreads();
+      row_sync();
     }
 
     // ---------------- inverse stage 1 and store ----------------
@@ -1083,15 +1113,15 @@ __device__ __forceinline__ void begin_after_previous()
 }
 
 // Standalone launch: one tile per CTA, or per cluster of CS CTAs.
-template <int LOGN, int MODE, int THREADS, int EPTW = 32>
-__global__ void __launch_bounds__(THREADS, (Sched<LOGN, THREADS, EPTW>::MINB)) rows_kernel(RowArgs a)
+template <int LOGN, int MODE, int THREADS, int EPTW = 32, bool FEW = false>
+__global__ void __launch_bounds__(THREADS, (FEW ? 1 : Sched<LOGN, THREADS, EPTW>::MINB)) rows_kernel(RowArgs a)
 {
   using S = Sched<LOGN, THREADS, EPTW>;
   begin_after_previous();
   if constexpr (S::CS > 1)
-    row_tile<LOGN, MODE, THREADS, EPTW>(a, blockIdx.x / S::CS, (int)cg::this_cluster().block_rank(), 0, true);
+    row_tile<LOGN, MODE, THREADS, EPTW, 0, FEW>(a, blockIdx.x / S::CS, (int)cg::this_cluster().block_rank(), 0, true);
   else
-    row_tile<LOGN, MODE, THREADS, EPTW>(a, blockIdx.x, 0, 0, true);
+    row_tile<LOGN, MODE, THREADS, EPTW, 0, FEW>(a, blockIdx.x, 0, 0, true);
 }
 
 }  // namespace fcb

@@ -28,6 +28,7 @@ struct KernelInfo
   long long tw_bytes = 0; // twiddle table size
   int ept = 32;          // samples per thread (the tables depend on it)
   long long resident_tiles = 0;  // CTAs (or clusters) resident at once, set by prepare_kernel
+  KernelInfo *few = nullptr;     // the kernel for calls whose rows are all resident at once in it
 };
 
 constexpr int kMin512 = 12;  // 512-thread variants exist for rows of 4096 samples and more
