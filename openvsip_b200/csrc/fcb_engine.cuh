@@ -1100,16 +1100,17 @@ __device__ __forceinline__ void row_tile(const RowArgs &a, long long tile, int r
   }
 }
 
-// Every kernel of the library that a call launches begins with these two, and is
-// launched with the programmatic-serialization attribute (see launch_kernel), so
-// that the launch of a call overlaps the end of the one before it: wait until the
-// work queued before this kernel is complete and visible, then let the next
-// kernel's CTAs take free places (they wait in turn).  Nothing may touch global
-// memory before the wait.
+// The kernels that calls launch begin with this and are launched with the
+// programmatic-serialization attribute (see launch_kernel), so that the launch of a
+// call overlaps the end of the one before it: wait until the work queued before this
+// kernel is complete and visible.  Nothing may touch global memory before the wait.
+// No launch_dependents: a next grid that takes free places while this one runs
+// slowed grids that fill part of the GPU (fast convolution of 300 rows of 4096,
+// back to back: 11.0 us against 8.3 when it starts as this one's CTAs exit, 10.3
+// without the attribute) and gained nothing elsewhere.
 __device__ __forceinline__ void begin_after_previous()
 {
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
 // Standalone launch: one tile per CTA, or per cluster of CS CTAs.
