@@ -126,16 +126,17 @@ MrConfig configure_rows(const MixedPlan &p, long long count, int sms)
   return best;
 }
 
-// Columns: C adjacent ones per CTA, so that accesses cover 8 C bytes side by side.  At least 4 (a 32-byte sector)
-// where they fit, more while two CTAs fit an SM and every SM has one.
+// Columns: C adjacent ones per CTA, so that accesses cover 8 C bytes side by side.  Up to 4 (a 32-byte sector) only as
+// many as bring the call down to one CTA an SM (100 columns of 7000: C = 1 15.3 us, 2 17.6, 4 24.6; 256 of 4096: 20.4,
+// 12.4, -), from there as many as leave every SM a CTA and room for two.
 MrConfig configure_cols(const MixedPlan &p, long long count, long long groups, int sms)
 {
+  auto grid = [&](int C) { return (count + C - 1) / C * groups; };
   int C = 1;
   while (C < 32 && C < count)
   {
     const long long smem = 16LL * C * p.n;
-    if (smem > kMrSmem) break;
-    if (C >= 4 && (smem > kMrSmem / 2 || (count + 2 * C - 1) / (2 * C) * groups < sms)) break;
+    if (smem > kMrSmem || (C < 4 ? grid(C) <= sms : smem > kMrSmem / 2 || grid(2 * C) < sms)) break;
     C *= 2;
   }
   // enough threads for one butterfly each, at most 256 where several CTAs share an SM

@@ -50,7 +50,7 @@ def test_fastconv_vector_and_matrix(oracle, rows, n):
 
 
 #       one column, one stage, partial last CTA, ragged, two columns per CTA, the longest, longer: through rows
-COLUMNS = [(13, 1), (2, 70), (756, 45), (1000, 67), (4096, 9), (8192, 5), (14336, 3), (16384, 3), (67, 5)]
+COLUMNS = [(13, 1), (2, 70), (756, 45), (1000, 67), (4096, 9), (4096, 130), (8192, 5), (14336, 3), (16384, 3), (67, 5)]
 
 
 @pytest.mark.parametrize("n,m", COLUMNS)
