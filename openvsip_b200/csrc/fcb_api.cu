@@ -54,8 +54,9 @@ struct fcb_plan_s
   MixedPlan *mxc = nullptr;
   float2 *twx = nullptr;           // W^k of the column length
   // 2-D FFT of other sizes (any dimensions the row plans support): a row plan
-  // of length cols, a transpose, a row plan of length rows on the transposed
-  // matrix, and a transpose back; scratch2 holds the transposed matrix.
+  // of length cols, then the column kernel; where the columns have none, a
+  // transpose, a row plan of length rows on the transposed matrix (scratch2), and
+  // a transpose back.
   bool general2d = false;
   fcb_plan sub2d[2] = {nullptr, nullptr};
   float2 *scratch2 = nullptr;
@@ -112,9 +113,10 @@ bool blue_length(long long n) { return n > 0 && n <= kMaxBlueN && (n & (n - 1)) 
 // columns left to the second pass: four of them (a 32-byte sector of each row) fit
 // its CTA.  Smallest matrix: against two transposing passes 4096 x 4096 measured
 // 179 -> 144 us, 8192 x 8192 917 -> 709, 1024 x 8192 106 -> 77, 2048 x 2048 45.4 ->
-// 40.4, but 1024 x 1024 14.9 -> 16.4 and 512 x 512 11.9 -> 12.2 us (the second
-// pass's stages take longer than one more row pass when both are a single wave).
-constexpr long long kCrossMaxRest = 4096, kCrossMinSamples = 1LL << 21;
+// 40.4, but 1024 x 1024 14.9 -> 16.4 and 2048 x 256 13.2 -> 13.8 us (the second
+// pass's stages take longer than one more row pass when both are a single wave);
+// from 4096 rows up also smaller ones (4096 x 256 18.7 -> 15.4, 4096 x 64 18.1 -> 16.7).
+constexpr long long kCrossMaxRest = 4096, kCrossMinSamples = 1LL << 21, kCrossMinRows = 4096;
 
 #define FCB_LENGTH_RULE "any length in [1, 32768], or a power of two up to 65536"
 
@@ -703,6 +705,8 @@ int exec_2d(fcb_plan p, const float2 *in, long long in_rs, float2 *out, long lon
   {
     const long long R = p->rows2d, C = p->cols2d;
     int rc = exec_device(p->sub2d[0], in, in_rs, p->scratch, C, R, 0, st);
+    if (!rc && !p->scratch2)  // the column kernel takes the rest
+      return mixed_transform(p->sub2d[1]->mx, true, p->scratch, C, out, out_rs, C, p->mode == kInv, p->scale, st);
     if (!rc) rc = launch_transpose(p->scratch, C, p->scratch2, R, R, C, st);        // scratch2 = scratch^T
     if (!rc) rc = exec_device(p->sub2d[1], p->scratch2, R, p->scratch2, R, C, 0, st);  // the columns, scaled
     if (!rc) rc = launch_transpose(p->scratch2, R, out, out_rs, C, R, st);
@@ -1423,9 +1427,13 @@ int fcb_plan_fft2d(long long rows, long long cols, int exponent, float scale, fc
   *plan = nullptr;
   if (exponent != FCB_FORWARD && exponent != FCB_INVERSE) return set_error(FCB_ERR_INVALID, "exponent must be -1 or +1");
   const int lr = log2_exact(rows), lc = log2_exact(cols);
-  if (lr < 6 || lr > 14 || lc < 6 || lc > 14)
+  // Small powers of two take the rows and then the columns too, up to columns of 1024: 1024 x 1024 / 512 x 512 /
+  // 256 x 2048 / 64 x 1024 14.8 / 11.9 / 13.3 / 12.4 us in two transposing passes (whose CTAs of 512 threads are few
+  // there), 12.8 / 8.3 / 8.7 / 6.2 this way, but 2048 x 256 13.2 / 15.7.  Taller ones: see kCrossMinSamples.
+  const bool small = rows * cols < kCrossMinSamples && rows <= 1024;
+  if (lr < 6 || lr > 14 || lc < 6 || lc > 14 || small)
   {
-    // other sizes: two row plans and two transposes (four passes)
+    // other sizes: a row plan and the column kernel, or two row plans and two transposes
     if (rows < 1 || cols < 1 || !fcb_supported_length(rows) || !fcb_supported_length(cols))
       return set_error(FCB_ERR_UNSUPPORTED, "2-D FFT dimensions %lld x %lld: each must be " FCB_LENGTH_RULE, rows,
                        cols);
@@ -1446,11 +1454,11 @@ int fcb_plan_fft2d(long long rows, long long cols, int exponent, float scale, fc
     if (e != cudaSuccess) rc = cuda_error(e, "cudaStreamCreate");
     p->stream = p->own_stream;
     if (!rc) rc = fcb_plan_fftm(cols, rows, exponent, 1.f, &p->sub2d[0]);
-    if (!rc) rc = fcb_plan_fftm(rows, cols, exponent, scale, &p->sub2d[1]);
+    if (!rc) rc = fcb_plan_fftm_cols(rows, cols, exponent, scale, &p->sub2d[1]);
     const size_t bytes = sizeof(float2) * (size_t)(rows * cols);
     if (!rc && (e = cudaMalloc(&p->scratch, bytes)) != cudaSuccess)
       rc = set_error(FCB_ERR_NOMEM, "2-D scratch: %s", cudaGetErrorString(e));
-    if (!rc && (e = cudaMalloc(&p->scratch2, bytes)) != cudaSuccess)
+    if (!rc && !fcb_supported_cols(rows) && (e = cudaMalloc(&p->scratch2, bytes)) != cudaSuccess)
       rc = set_error(FCB_ERR_NOMEM, "2-D scratch: %s", cudaGetErrorString(e));
     if (rc) { plan_free(p); return rc; }
     *plan = p;
@@ -1467,7 +1475,8 @@ int fcb_plan_fft2d(long long rows, long long cols, int exponent, float scale, fc
   if (!rc)
   {
     const CrossKernel *kx = cross_kernel(lc, mode == kInv);
-    if (kx && rows / kx->radix <= kCrossMaxRest && rows * cols >= kCrossMinSamples)
+    if (kx && rows / kx->radix <= kCrossMaxRest &&
+        (rows * cols >= kCrossMinSamples || rows >= kCrossMinRows))
     {
       p->kx = kx;
       p->k = &kx->k;
