@@ -21,7 +21,7 @@ ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden",
          f"-I{os.path.join(ROOT, 'include')}", f"-I{CSRC}"]
 
-SOURCES = ["fcb_rows_conv.cu", "fcb_rows_fwd.cu", "fcb_rows_inv.cu", "fcb_rows_r2c.cu",
+SOURCES = ["fcb_rows_conv.cu", "fcb_rows_coefs.cu", "fcb_rows_fwd.cu", "fcb_rows_inv.cu", "fcb_rows_r2c.cu",
            "fcb_rows_c2r.cu", "fcb_rows_cross.cu", "fcb_batch.cu", "fcb_mixed_conv.cu", "fcb_mixed_rows.cu",
            "fcb_mixed_cols.cu", "fcb_mixed.cu", "fcb200.cu",
            "fcb_api.cu", "fcb_bluestein.cu", "fcb_real.cu", "fcb_hostcopy.cu"]

@@ -338,6 +338,16 @@ const KernelInfo *real_kernel(int logn, bool inverse, const KernelInfo *like)
   return v < 0 || !tab[inverse][logn][v].fn ? nullptr : &tab[inverse][logn][v];
 }
 
+const KernelInfo *coefs_kernel(int logn, const KernelInfo *like)
+{
+  static KernelInfo tab[kMaxLogN + 1][kVariants];
+  static std::once_flag once;
+  std::call_once(once, [] { rows_table_coefs(tab); });
+  if (logn < 1 || logn > kMaxLogN || !like) return nullptr;
+  const int v = variant_id(logn, like->ept == 64 ? -like->threads : like->threads);
+  return v < 0 || !tab[logn][v].fn ? nullptr : &tab[logn][v];
+}
+
 int set_variant(int logn, int mode, int threads)
 {
   init_table();

@@ -396,12 +396,15 @@ __device__ __forceinline__ void prefetch_l2_bulk(const void *p, uint32_t bytes)
 // kR2C and kC2R are the transforms of real rows of 2N samples, read or written
 // as N complex ones: kR2C splits Z into the N + 1 bins of the half spectrum as
 // it stores, kC2R merges the half spectrum into Z as it loads.
+// kCoefs is the fused fast convolution with a replica row for every data row (a
+// matrix of coefficients): the replica comes from HBM too, and is fetched ahead.
 // kFwdCross and kInvCross are the row pass of a 2-D FFT that takes the column
 // transforms' first stage along: the rows of a CTA lie a.cross rows apart (in
 // groups of G, see cross_radix) and are combined by a radix-G step before they
 // are stored, so that the column pass is left with columns of 1 / G the length
 // and can take 64 to 128 bytes of each row at a time.
-enum Mode { kFwd = 0, kInv = 1, kFastconv = 2, kChirpconv = 3, kR2C = 4, kC2R = 5, kFwdCross = 6, kInvCross = 7 };
+enum Mode { kFwd = 0, kInv = 1, kFastconv = 2, kChirpconv = 3, kR2C = 4, kC2R = 5, kFwdCross = 6, kInvCross = 7,
+            kCoefs = 8 };
 
 // Rows that a cross pass combines, of the rows its CTA holds.
 template <class S>
@@ -495,7 +498,7 @@ __device__ __forceinline__ void row_tile(const RowArgs &a, long long tile, int r
   constexpr int SIGN = (MODE == kInv || MODE == kC2R || MODE == kInvCross) ? +1 : -1;  // direction of the first pass
   constexpr bool CHIRP = MODE == kChirpconv, CROSS = MODE == kFwdCross || MODE == kInvCross;
   // the transform structure
-  constexpr int MD = CHIRP ? kFastconv : (MODE == kR2C || MODE == kFwdCross) ? kFwd
+  constexpr int MD = CHIRP || MODE == kCoefs ? kFastconv : (MODE == kR2C || MODE == kFwdCross) ? kFwd
                    : (MODE == kC2R || MODE == kInvCross) ? kInv : MODE;
   constexpr int LH1 = ilog2(S::H1);
   constexpr bool CL = S::CS > 1;
@@ -618,6 +621,11 @@ __device__ __forceinline__ void row_tile(const RowArgs &a, long long tile, int r
       for (int j = 0; j < S::EPT; ++j)
         x[j] = active ? __ldg(src + tr + S::TPR * j) : make_float2(0.f, 0.f);
     }
+    // A replica row of its own is first read in the last forward stage, a few
+    // entries at a time: from HBM one memory latency after another.  Bring it into L2
+    // behind the input loads.
+    if constexpr (MODE == kCoefs)
+      if (tr == 0 && active) prefetch_l2_bulk(a.rep + row * a.rep_rs, 16u * S::HALF);
     // With this tile's loads in flight, prefetch into L2 the input of the tile
     // `ahead` tiles later (about half a resident wave), so that it streams in
     // from HBM while this tile computes.  Straight-line code (a few lines per

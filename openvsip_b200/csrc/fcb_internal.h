@@ -43,6 +43,7 @@ constexpr int kVariants = 4;
 void rows_table_fwd(KernelInfo (*tab)[kVariants]);
 void rows_table_inv(KernelInfo (*tab)[kVariants]);
 void rows_table_conv(KernelInfo (*tab)[kVariants]);
+void rows_table_coefs(KernelInfo (*tab)[kVariants]);
 void rows_table_r2c(KernelInfo (*tab)[kVariants]);
 void rows_table_c2r(KernelInfo (*tab)[kVariants]);
 const KernelInfo *kernel_info(int logn, int mode);
@@ -55,6 +56,9 @@ const KernelInfo *chirp_kernel(int logn, const KernelInfo *like);
 // split of rows that span a cluster: measured 125 us against 89 us for two passes
 // over 256 rows of 65536, each bin pair reading two slots of other CTAs).
 const KernelInfo *real_kernel(int logn, bool inverse, const KernelInfo *like);
+// Fused kernel for a replica row per data row, in the same variant as `like`; NULL
+// where there is none (rows that span a cluster).
+const KernelInfo *coefs_kernel(int logn, const KernelInfo *like);
 // Row pass of a 2-D transform that combines `radix` rows (fcb_rows_cross.cu):
 // rows of 64 .. 8192 samples.
 struct CrossKernel

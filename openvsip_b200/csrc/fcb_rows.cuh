@@ -15,8 +15,8 @@ KernelInfo rows_info()
 {
   using S = Sched<LOGN, T, EPTW>;
   KernelInfo k;
-  // the split of real rows has no cluster form (entry left empty)
-  if constexpr (MODE != kR2C || S::CS == 1) k.fn = (const void *)&rows_kernel<LOGN, MODE, T, EPTW, FEW>;
+  // the split of real rows and the replica-per-row form have no cluster form (entry left empty)
+  if constexpr ((MODE != kR2C && MODE != kCoefs) || S::CS == 1) k.fn = (const void *)&rows_kernel<LOGN, MODE, T, EPTW, FEW>;
   k.ept = EPTW;
   k.threads = T;
   k.cluster = S::CS;
@@ -26,7 +26,7 @@ KernelInfo rows_info()
   // The kernel for calls of few rows (same tables, same arithmetic), for the variants that are
   // the defaults: the FEW form of the same CTA up to 8192 samples; from 16384 up, where a CTA of
   // 512 threads fills an SM anyway, twice as many CTAs of 256 threads for a row.
-  if constexpr (!FEW && EPTW == 32)
+  if constexpr (!FEW && EPTW == 32 && MODE != kCoefs)
   {
     constexpr bool same = (T == 128 && LOGN <= 12) || (T == 256 && (LOGN < kMin128 || LOGN == 13));
     constexpr bool split = T == 512 && LOGN >= 14 && MODE != kR2C;

@@ -37,3 +37,17 @@ def test_rows_do_not_depend_on_their_number(oracle, n):
         for rows in (1, 18, 37, 75, 149, 297):
             assert torch.equal(f(real[:rows], torch.empty_like(spec[:rows])), spec[:rows]), (n, rows)
             assert torch.equal(b(spec[:rows], torch.empty_like(back[:rows])), back[:rows]), (n, rows)
+
+
+@pytest.mark.parametrize("n,many", [(512, 5000), (4096, 1300), (16384, 400), (32768, 80)])
+def test_matrix_of_coefficients_equals_its_rows(n, many):
+    # more rows than are resident at once take the kernel that fetches replica rows ahead
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(n)
+    x, w = (torch.view_as_complex(torch.randn(many, n, 2, generator=g, device="cuda")) for _ in range(2))
+    full = Fastconv(w, many)(x)
+    for lo, hi in ((0, 3), (many // 2, many // 2 + 100), (many - 2, many)):
+        hi = min(hi, many)
+        part = Fastconv(w[lo:hi], hi - lo)(x[lo:hi])
+        assert torch.equal(part, full[lo:hi])
+    assert torch.equal(Fastconv(w[5], 2)(x[5:7])[:1], full[5:6])
