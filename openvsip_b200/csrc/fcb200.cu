@@ -422,11 +422,12 @@ int launch_rows(const KernelInfo *k, long long rows, const RowArgs &args, cudaSt
   RowArgs a = args;
   if (a.ahead < 0) a.ahead = (k->resident_tiles + 1) / 2;  // half a resident wave ahead (measured best)
   void *params[] = {&a};
-  return launch_kernel(k->fn, dim3((unsigned)ctas), k->threads, k->cluster, k->smem, params, st, "row kernel launch");
+  return launch_kernel(k->fn, dim3((unsigned)ctas), k->threads, k->cluster, k->smem, params, st, "row kernel launch",
+                       k->overlapped);
 }
 
 int launch_kernel(const void *fn, dim3 grid, int threads, int cluster, size_t smem, void **params, cudaStream_t st,
-                  const char *what)
+                  const char *what, bool overlapped)
 {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
@@ -447,14 +448,17 @@ int launch_kernel(const void *fn, dim3 grid, int threads, int cluster, size_t sm
   // a captured launch stays an ordinary graph node: programmatic edges would not
   // survive every caller's capture queries
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone)
+  if (overlapped && cudaStreamIsCapturing(st, &cap) != cudaSuccess)
+  {
+    cudaGetLastError();
+    overlapped = false;
+  }
+  if (overlapped && cap == cudaStreamCaptureStatusNone)
   {
     attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[cfg.numAttrs].val.programmaticStreamSerializationAllowed = 1;
     ++cfg.numAttrs;
   }
-  else
-    cudaGetLastError();
   const cudaError_t e = cudaLaunchKernelExC(&cfg, fn, params);
   return e == cudaSuccess ? FCB_OK : cuda_error(e, what);
 }

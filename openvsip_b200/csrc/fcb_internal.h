@@ -27,6 +27,7 @@ struct KernelInfo
   int smem = 0;          // dynamic shared memory per CTA, bytes
   long long tw_bytes = 0; // twiddle table size
   int ept = 32;          // samples per thread (the tables depend on it)
+  bool overlapped = true;        // the launch overlaps the kernel before (begin_after_previous)
   long long resident_tiles = 0;  // CTAs (or clusters) resident at once, set by prepare_kernel
   KernelInfo *few = nullptr;     // the kernel for calls whose rows are all resident at once in it
 };
@@ -72,10 +73,11 @@ int set_variant(int logn, int mode, int threads);
 const KernelInfo *kernel_variant(int logn, int mode, int threads);
 int get_variant(int logn, int mode);
 int prepare_kernel(const KernelInfo *k);
-// Launches a kernel that starts with begin_after_previous(), in clusters of `cluster`
-// CTAs, so that its launch overlaps the end of the kernel before it in the stream.
+// Launches a kernel in clusters of `cluster` CTAs; one that starts with
+// begin_after_previous() (overlapped) so that its launch overlaps the end of the
+// kernel before it in the stream.
 int launch_kernel(const void *fn, dim3 grid, int threads, int cluster, size_t smem, void **params, cudaStream_t st,
-                  const char *what);
+                  const char *what, bool overlapped = true);
 int launch_rows(const KernelInfo *k, long long rows, const RowArgs &args, cudaStream_t st);
 
 int build_twiddles(int logn, int ept, float4 **out, cudaStream_t st);

@@ -80,16 +80,9 @@ struct MrArgs
   long long rep_bs;
   float scale;             // transform: output scale
   int inverse;             // transform: exchange re and im on the way in and out
-  // chirp convolution (Bluestein rows): in[k] * cin[r * cin_bs + k] for k < n_in and 0 beyond;
-  // outputs k < n_out only, times cout[k] when set
-  const float2 *cin;
-  long long cin_bs;
-  int n_in;
-  const float2 *cout;
-  int n_out;
 };
 
-enum MrKind { kMrTransform = 0, kMrConv = 1, kMrChirp = 2 };
+enum MrKind { kMrTransform = 0, kMrConv = 1 };
 
 // ---------------------------------------------------------------------------
 // cos and sin of 2 pi k / R, evaluated by the compiler in double (Taylor series
@@ -316,35 +309,15 @@ __global__ void __launch_bounds__(MAXT, MINB) mixed_kernel(const __grid_constant
     constexpr int R = decltype(rc)::value;
     const float2 *p = a.in + (COL ? blockIdx.y * a.in_gs : 0) + (r0 + c) * a.in_bs + b * a.in_es;
     const long long step = s.S * a.in_es;
-    if constexpr (KIND == kMrChirp)
-    {
-      const float2 *m = a.cin + (r0 + c) * a.cin_bs + b;
 #pragma unroll
-      for (int r = 0; r < R; ++r)
-        x[r] = b + s.S * r < a.n_in ? mr_cmul(__ldg(p + r * step), __ldg(m + s.S * r)) : make_float2(0.f, 0.f);
-    }
-    else
-    {
-#pragma unroll
-      for (int r = 0; r < R; ++r) x[r] = swap_if(__ldg(p + r * step), inv);
-    }
+    for (int r = 0; r < R; ++r) x[r] = swap_if(p[r * step], inv);
   };
   // natural-order outputs of the last inverse stage (re and im exchanged)
   auto store_conv = [&](const MrStage &s, int c, int b, auto rc, const float2 *x) {
     constexpr int R = decltype(rc)::value;
     float2 *p = a.out + (r0 + c) * a.out_bs + b;
 #pragma unroll
-    for (int r = 0; r < R; ++r)
-    {
-      const int k = b + s.S * r;
-      const float2 v = make_float2(x[r].y, x[r].x);
-      if constexpr (KIND == kMrChirp)
-      {
-        if (k < a.n_out) p[s.S * r] = a.cout ? mr_cmul(v, __ldg(a.cout + k)) : v;
-      }
-      else
-        p[s.S * r] = v;
-    }
+    for (int r = 0; r < R; ++r) p[s.S * r] = make_float2(x[r].y, x[r].x);
   };
   auto times_replica = [&](const MrStage &s, int c, int b, auto rc, float2 *x) {
     constexpr int R = decltype(rc)::value;

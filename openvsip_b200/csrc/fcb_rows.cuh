@@ -18,6 +18,7 @@ KernelInfo rows_info()
   // the split of real rows and the replica-per-row form have no cluster form (entry left empty)
   if constexpr ((MODE != kR2C && MODE != kCoefs) || S::CS == 1) k.fn = (const void *)&rows_kernel<LOGN, MODE, T, EPTW, FEW>;
   k.ept = EPTW;
+  k.overlapped = overlapped_rows(EPTW);
   k.threads = T;
   k.cluster = S::CS;
   k.rows_per_cta = S::ROWS;

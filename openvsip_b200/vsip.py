@@ -291,11 +291,12 @@ class Fftm(_Plan):
         check(plan(n, count, self.exponent, self.scale, ctypes.byref(h)))
         self._handle = h
         self._n = n
-        self._col_kernel = self.axis == col and bool(lib().fcb_supported_cols(n))
         # Few columns of a long power of two are quicker as rows (the row kernel spreads a row
         # over more threads): 64 of 4096 9.7 us against 11.9, 64 of 8192 13.9 against 21.3; 128 of
-        # 4096 the same, 256 of 4096 18.8 against 12.4, of 8192 33 against 22.6.
-        self._col_min = 129 if n >= 4096 and n & (n - 1) == 0 else 1
+        # 4096 the same, 256 of 4096 18.8 against 12.4, of 8192 33 against 22.6.  By the plan's
+        # count, so that a column's result does not depend on how many a call passes.
+        few = n >= 4096 and n & (n - 1) == 0 and count <= 128
+        self._col_kernel = self.axis == col and not few and bool(lib().fcb_supported_cols(n))
 
     def __call__(self, inp, out=None):
         """By reference: ``fftm(in, out)``; ``fftm(in)`` returns a new result (by value)."""
@@ -311,10 +312,9 @@ class Fftm(_Plan):
         return self._exec(inout, inout)
 
     def _columns(self, inp, out):
-        kernel = self._col_kernel and len(inp.shape) == 2 and inp.shape[1] >= self._col_min
-        if kernel and type(inp) is not np.ndarray and self._device_call(_COLS, inp, out, self._n, self.cols):
+        if self._col_kernel and type(inp) is not np.ndarray and self._device_call(_COLS, inp, out, self._n, self.cols):
             return out
-        a = _plain_matrix(inp, False) if kernel else None
+        a = _plain_matrix(inp, False) if self._col_kernel else None
         b = _plain_matrix(out, True) if a else None
         if not (a and b and a[1:3] == b[1:3] and a[1] == self._n and a[2] <= self.cols and a[4] == b[4]
                 and _same_or_apart(a, b)):
