@@ -38,7 +38,7 @@
  *                                 persistent launch.
  *
  * Lengths: Fftm, fast-convolution and replica plans take any length from 1 to
- * 32768 (lengths that are not powers of two run Bluestein's algorithm) and
+ * 32768 (mixed radix or Bluestein's algorithm where not a power of two) and
  * powers of two up to 65536; the batch entry points take powers of two from
  * 256 to 32768; the 2-D plans take any supported length per dimension.
  */
