@@ -77,7 +77,8 @@ struct fcb_plan_s
   // any such length: the mixed-radix kernel.
   MixedPlan *mx = nullptr;
   float2 *mx_rep = nullptr;                    // fastconv: replica table(s), last-stage order
-  float2 *cstage = nullptr;                    // host column calls: device copy of a block of columns
+  std::mutex cols_mu;                          // host column calls: one at a time has the block below
+  float2 *cstage = nullptr;                    // device copy of a block of columns
   long long cstage_cols = 0;
   // Real-input rows of n = rn samples: 1 = real -> complex (n/2 + 1 outputs),
   // 2 = complex -> real.  Even n: a length-n/2 complex plan plus the split /
@@ -1151,7 +1152,9 @@ int fcb_exec_cols(fcb_plan p, const fcb_cf32 *in, long long in_rs, fcb_cf32 *out
   float2 *o2 = reinterpret_cast<float2 *>(out);
   if (where == FCB_DEVICE)
     return mixed_transform(p->mx, true, i2, in_rs, o2, out_rs, cols, p->mode == kInv, p->scale, p->stream);
-  // host columns: blocks of them through one device buffer
+  // host columns: blocks of them through one device buffer, which threads that share the plan
+  // take in turn (as they take the shared pinned buffers of the row calls)
+  std::lock_guard<std::mutex> turn(p->cols_mu);
   const long long n = p->n, chunk = std::min(cols, std::max<long long>(1, (long long)(4 * stage_bytes()) / (8 * n)));
   if (p->cstage_cols < chunk)
   {
