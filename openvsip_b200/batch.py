@@ -44,7 +44,7 @@ class Batch:
         """Make a replica resident; numpy (host) or CUDA tensor (device), complex64."""
         rid = ctypes.c_int()
         if type(replica).__module__.startswith("torch"):
-            r = replica.contiguous().reshape(-1)
+            r = replica.resolve_conj().resolve_neg().contiguous().reshape(-1)
             check(lib().fcb_batch_add_replica(self._h, ctypes.c_void_p(r.data_ptr()), r.numel(), _KINDS[kind],
                                               _lib.FCB_DEVICE, ctypes.byref(rid)))
         else:
@@ -64,6 +64,8 @@ class Batch:
             for t in (x, y):
                 if not (type(t).__module__.startswith("torch") and t.is_cuda and t.dim() == 2 and t.stride(1) == 1):
                     raise TypeError("batch jobs take 2-D CUDA complex64 tensors with unit-stride rows")
+                if t.is_conj() or t.is_neg():  # the job table holds memory, which run() reads each time
+                    raise TypeError("batch jobs take tensors that hold their values: resolve_conj(), resolve_neg()")
             arr[i].in_ = x.data_ptr()
             arr[i].in_rs = x.stride(0) if x.shape[0] > 1 else x.shape[1]
             arr[i].out = y.data_ptr()

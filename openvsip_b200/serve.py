@@ -106,6 +106,7 @@ class Server:
     def submit(self, x, replica: int) -> Request:
         if not (0 <= replica < self.nreplicas):
             raise ValueError("unknown replica id")
+        x = x.resolve_conj().resolve_neg()  # a lazy conjugate's memory holds the values of another tensor
         ready = self.torch.cuda.Event()
         ready.record()
         r = Request(x, replica, ready)

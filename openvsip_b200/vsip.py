@@ -108,6 +108,26 @@ def _desc(x, writable: bool, real: bool = False):
     return a.ctypes.data, a.shape[0], a.shape[1], rs, _lib.FCB_HOST
 
 
+def _lazy(x) -> bool:
+    """A tensor whose memory does not hold its values: torch's conj() and views of
+    its imaginary part only mark the conjugate or the negative."""
+    return type(x) is not np.ndarray and _is_torch(x) and (x.is_conj() or x.is_neg())
+
+
+def _held(x):
+    """x with its values in memory."""
+    return x.resolve_conj().resolve_neg()
+
+
+def _call_held(call, inp, out):
+    """call(inp, out) where either is lazy: on the input's values, the output
+    written back the way torch writes such a tensor."""
+    if not _lazy(out):
+        call(_held(inp), out)
+        return out
+    y = _torch_mod().empty(out.shape, dtype=out.dtype, device=out.device)
+    call(_held(inp), y)
+    return out.copy_(y)
 
 
 def _empty_like(x):
@@ -129,8 +149,7 @@ def _transposed(x):
     """Contiguous transpose: the column-major copy the reference's DDA layer makes
     for a column-axis Fftm (query_layout asks for tuple<1,0,2>)."""
     if _is_torch(x):
-        # a lazy conjugate would survive contiguous() where no copy is needed (one column)
-        return x.t().resolve_conj().resolve_neg().contiguous()
+        return _held(x.t()).contiguous()  # a lazy conjugate would survive where no copy is needed (one column)
     return np.ascontiguousarray(x.T)
 
 
@@ -244,6 +263,8 @@ class _Plan:
             raise ValueError(f"row length {c} != planned {n}")
         if iw != ow:
             raise ValueError("input and output must both be host arrays or both device tensors")
+        if _lazy(inp) or _lazy(out):
+            return _call_held(lambda a, b: self._exec(a, b, wait), inp, out)
         self._bind_stream(iw)
         fn = lib().fcb_exec if wait else lib().fcb_exec_async
         check(fn(self._handle, ctypes.c_void_p(ip), irs, ctypes.c_void_p(op), ors, r, iw))
@@ -381,6 +402,8 @@ class FftmReal(_Plan):
             raise ValueError(f"shapes {(r, c)} -> {(r2, c2)} do not match n={self.n}")
         if iw != ow:
             raise ValueError("input and output must both be host arrays or both device tensors")
+        if _lazy(inp) or _lazy(out):
+            return _call_held(self._rows, inp, out)
         self._bind_stream(iw)
         fn = lib().fcb_exec_r2c if fwd else lib().fcb_exec_c2r
         check(fn(self._handle, ctypes.c_void_p(ip), irs, ctypes.c_void_p(op), ors, r, iw))
@@ -424,6 +447,9 @@ class Fastconv(_Plan):
         if not _is_torch(weights):
             weights = np.ascontiguousarray(weights, dtype=np.complex64)
         wp, wr, wc, wrs, ww = _desc(weights, False)
+        if _lazy(weights):
+            weights = _held(weights)
+            wp, wr, wc, wrs, ww = _desc(weights, False)
         self.rows, self.cols = int(rows), int(wc)
         self._n = self.cols
         self.replica_rows = wr
@@ -453,10 +479,11 @@ def vmmul(v, m, out=None):
         out = torch.empty_like(m)
     mp, r, c, mrs, _ = _desc(m, False)
     op, r2, c2, ors, _ = _desc(out, True)
-    if not v.is_contiguous():
-        v = v.contiguous()
+    v = _held(v).contiguous()
     if v.numel() != c or (r2, c2) != (r, c):
         raise ValueError("shape mismatch")
+    if _lazy(m) or _lazy(out):
+        return _call_held(lambda a, b: vmmul(v, a, b), m, out)
     stream = _stream_handle()
     check(lib().fcb_vmmul_rows(ctypes.c_void_p(v.data_ptr()), ctypes.c_void_p(mp), mrs, ctypes.c_void_p(op),
                                ors, r, c, ctypes.c_void_p(stream)))
@@ -468,7 +495,7 @@ def replica_spectrum(replica, matched: bool = True):
     import torch
     if not (_is_torch(replica) and replica.is_cuda):
         raise TypeError("pass a CUDA complex64 tensor")
-    r = replica.contiguous().reshape(-1)
+    r = _held(replica).contiguous().reshape(-1)
     out = torch.empty_like(r)
     torch.cuda.current_stream().synchronize()
     check(lib().fcb_replica_spectrum(ctypes.c_void_p(r.data_ptr()), r.numel(), int(bool(matched)),
