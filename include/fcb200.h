@@ -146,7 +146,9 @@ FCB_API int fcb_plan_fft2d(long long rows, long long cols, int exponent, float s
 /* Fused fast-convolution plan: y = IFFT(R .* FFT(x)) / n per row.
  * replica: replica_rows rows (1 = one vector shared by all rows, or one per
  * data row) of n samples at row stride replica_rs, kind fcb_replica_kind,
- * located at `where`.  The plan keeps the spectrum resident on the device. */
+ * located at `where`.  The plan keeps the spectrum resident on the device.  A
+ * device replica is read on a stream of the plan's own during this call: what
+ * writes it must be complete. */
 FCB_API int fcb_plan_fastconv(long long n, long long rows_max, const fcb_cf32 *replica,
                       long long replica_rows, long long replica_rs,
                       int replica_kind, int where, fcb_plan *plan);
@@ -271,7 +273,8 @@ typedef struct
  * thread, 32768 on clusters of two CTAs), or 0 for the default (512). */
 FCB_API int fcb_batch_create(int threads, fcb_batch *batch);
 /* Keep a replica resident on the device (spectrum built in FP64 for the time
- * kinds); returns its id. */
+ * kinds); returns its id.  A device replica is read on a stream of the batch's
+ * own during this call: what writes it must be complete. */
 FCB_API int fcb_batch_add_replica(fcb_batch batch, const fcb_cf32 *replica, long long n,
                                   int replica_kind, int where, int *id);
 /* Define the job list (copied).  order bit 0: 0 = longest rows first (default

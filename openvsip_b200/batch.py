@@ -18,6 +18,7 @@ import numpy as np
 
 from . import _lib
 from ._lib import FcbJob, check, lib
+from .vsip import _held, _settle
 
 _KINDS = {"spectrum": _lib.FCB_REPLICA_SPECTRUM, "time": _lib.FCB_REPLICA_TIME,
           "matched": _lib.FCB_REPLICA_TIME_MATCHED}
@@ -44,7 +45,9 @@ class Batch:
         """Make a replica resident; numpy (host) or CUDA tensor (device), complex64."""
         rid = ctypes.c_int()
         if type(replica).__module__.startswith("torch"):
-            r = replica.resolve_conj().resolve_neg().contiguous().reshape(-1)
+            r = _held(replica).contiguous().reshape(-1)
+            if r.is_cuda:
+                _settle(r)  # the batch reads it on its own stream
             check(lib().fcb_batch_add_replica(self._h, ctypes.c_void_p(r.data_ptr()), r.numel(), _KINDS[kind],
                                               _lib.FCB_DEVICE, ctypes.byref(rid)))
         else:

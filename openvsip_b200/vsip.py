@@ -114,6 +114,15 @@ def _lazy(x) -> bool:
     return type(x) is not np.ndarray and _is_torch(x) and (x.is_conj() or x.is_neg())
 
 
+def _settle(x) -> None:
+    """Wait for the work queued on the current torch stream, which may still be
+    writing the CUDA tensor x: a plan reads its weights on a stream of its own.
+    (Not while that stream is being captured: its work has not run either way.)"""
+    cuda = _torch_mod().cuda
+    if not cuda.is_current_stream_capturing():
+        cuda.current_stream(x.device).synchronize()
+
+
 def _held(x):
     """x with its values in memory."""
     return x.resolve_conj().resolve_neg()
@@ -450,6 +459,8 @@ class Fastconv(_Plan):
         if _lazy(weights):
             weights = _held(weights)
             wp, wr, wc, wrs, ww = _desc(weights, False)
+        if ww == _lib.FCB_DEVICE:
+            _settle(weights)
         self.rows, self.cols = int(rows), int(wc)
         self._n = self.cols
         self.replica_rows = wr
@@ -497,7 +508,7 @@ def replica_spectrum(replica, matched: bool = True):
         raise TypeError("pass a CUDA complex64 tensor")
     r = _held(replica).contiguous().reshape(-1)
     out = torch.empty_like(r)
-    torch.cuda.current_stream().synchronize()
+    _settle(r)
     check(lib().fcb_replica_spectrum(ctypes.c_void_p(r.data_ptr()), r.numel(), int(bool(matched)),
                                      ctypes.c_void_p(out.data_ptr())))
     return out
