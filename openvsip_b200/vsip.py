@@ -383,6 +383,7 @@ class FftmReal(_Plan):
         h = ctypes.c_void_p()
         check(lib().fcb_plan_fftm_real(self.n, self.count, self.exponent, self.scale, ctypes.byref(h)))
         self._handle = h
+        self._n = self.cols
 
     def output_shape(self):
         if self.exponent == _lib.FCB_INVERSE:
