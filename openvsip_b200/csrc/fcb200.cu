@@ -372,39 +372,53 @@ int get_variant(int logn, int mode)
   return kVariantValue[g_variant[logn][mode]];
 }
 
-int prepare_kernel(const KernelInfo *k)
+// Sets up a kernel for launches and counts its CTAs (or clusters) resident at once.
+// by_cluster: of a kernel in clusters, one CTA an SM.
+static int prepare_one(const KernelInfo *k, bool by_cluster)
 {
   // Idempotent; cheap after the first call per device.
   cudaError_t e = cudaFuncSetAttribute(k->fn, cudaFuncAttributeMaxDynamicSharedMemorySize, k->smem);
   if (e != cudaSuccess) return cuda_error(e, "cudaFuncSetAttribute(smem)");
-  // tiles resident at once: the L2 prefetch distance, and the bound of a call of few rows
-  int dev = 0, sms = 0, per_sm = 0;
+  int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k->fn, k->threads, k->smem);
-  if (e != cudaSuccess) return cuda_error(e, "occupancy query");
-  const_cast<KernelInfo *>(k)->resident_tiles = (long long)sms * (per_sm > 0 ? per_sm : 1) / k->cluster;
-  if (!k->few) return FCB_OK;
-  const int rc = prepare_kernel(k->few);
-  if (rc || k->few->cluster == 1) return rc;
+  if (!by_cluster)
+  {
+    int per_sm = 0;
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k->fn, k->threads, k->smem);
+    if (e != cudaSuccess) return cuda_error(e, "occupancy query");
+    k->resident_tiles = (long long)sms * (per_sm > 0 ? per_sm : 1) / k->cluster;
+    return FCB_OK;
+  }
   // clusters lie within a GPC: fewer fit than the SM count says
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(sms / k->few->cluster * k->few->cluster));
-  cfg.blockDim = dim3(k->few->threads);
-  cfg.dynamicSmemBytes = k->few->smem;
+  cfg.gridDim = dim3((unsigned)(sms / k->cluster * k->cluster));
+  cfg.blockDim = dim3(k->threads);
+  cfg.dynamicSmemBytes = k->smem;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = k->few->cluster;
+  attr[0].val.clusterDim.x = k->cluster;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   int clusters = 0;
-  e = cudaOccupancyMaxActiveClusters(&clusters, k->few->fn, &cfg);
-  if (e != cudaSuccess) return cuda_error(e, "cluster occupancy query");
-  // one CTA an SM: with two, the ordinary kernel's row is as short
-  k->few->resident_tiles = std::min(clusters, sms / k->few->cluster);
+  if (cudaOccupancyMaxActiveClusters(&clusters, k->fn, &cfg) != cudaSuccess)
+  {
+    cudaGetLastError();
+    clusters = 0;  // not known: the ordinary kernel takes every call
+  }
+  k->resident_tiles = std::min(clusters, sms / k->cluster);
   return FCB_OK;
+}
+
+// The resident counts are the L2 prefetch distance, and the bound of a call of few rows
+// (there one CTA an SM: with two, the ordinary kernel's row is as short).  They are stored
+// once they are final: another thread's calls may be reading them.
+int prepare_kernel(const KernelInfo *k)
+{
+  const int rc = prepare_one(k, false);
+  return rc || !k->few ? rc : prepare_one(k->few, k->few->cluster > 1);
 }
 
 int launch_rows(const KernelInfo *k, long long rows, const RowArgs &args, cudaStream_t st)

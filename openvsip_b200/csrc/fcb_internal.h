@@ -3,6 +3,7 @@
 
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstddef>
 
 namespace fcb {
@@ -18,6 +19,21 @@ struct SchedRT
 };
 SchedRT sched_rt(int logn, int ept = 32);
 
+// A number that every plan's creation stores (always the same one) and every call reads.
+struct SharedCount
+{
+  std::atomic<long long> v{0};
+  SharedCount() = default;
+  SharedCount(const SharedCount &o) : v(o.v.load(std::memory_order_relaxed)) {}
+  SharedCount &operator=(const SharedCount &o) { return *this = (long long)o; }
+  SharedCount &operator=(long long n)
+  {
+    v.store(n, std::memory_order_relaxed);
+    return *this;
+  }
+  operator long long() const { return v.load(std::memory_order_relaxed); }
+};
+
 struct KernelInfo
 {
   const void *fn = nullptr;
@@ -28,8 +44,8 @@ struct KernelInfo
   long long tw_bytes = 0; // twiddle table size
   int ept = 32;          // samples per thread (the tables depend on it)
   bool overlapped = true;        // the launch overlaps the kernel before (begin_after_previous)
-  long long resident_tiles = 0;  // CTAs (or clusters) resident at once, set by prepare_kernel
-  KernelInfo *few = nullptr;     // the kernel for calls whose rows are all resident at once in it
+  mutable SharedCount resident_tiles;  // CTAs (or clusters) resident at once, set by prepare_kernel
+  const KernelInfo *few = nullptr;     // the kernel for calls whose rows are all resident at once in it
 };
 
 constexpr int kMin512 = 12;  // 512-thread variants exist for rows of 4096 samples and more

@@ -34,7 +34,7 @@ KernelInfo rows_info()
     if constexpr (same || split)
     {
       static const KernelInfo few = rows_info<LOGN, MODE, split ? 256 : T, 32, true>();
-      k.few = const_cast<KernelInfo *>(&few);
+      k.few = &few;
     }
   }
   return k;
