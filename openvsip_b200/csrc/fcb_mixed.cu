@@ -8,8 +8,8 @@
 
 #include <algorithm>
 #include <atomic>
+#include <memory>
 #include <new>
-#include <vector>
 
 namespace fcb {
 
@@ -49,11 +49,17 @@ float dft_cost(int R)
 // twiddles per sample, about the issue slots of 16 operations).
 constexpr float kPassCost = 16.f;
 
-// Radices of n with the least cost, in ascending order of their share of two: the last stage reads R adjacent samples
-// per thread, which is free of bank conflicts only for odd R.
-bool factor(int n, int max_stages, std::vector<int> &best)
+struct Radices
 {
-  std::vector<int> cur;
+  int r[kMrStages];
+  int count = 0;
+};
+
+// Radices of n with the least cost, in descending order of their share of two: the last stage reads R adjacent samples
+// per thread, which is free of bank conflicts only for odd R.
+bool factor(int n, Radices &best)
+{
+  Radices cur;
   float best_cost = 1e30f;
   auto rec = [&](auto &&self, int left, int from, float cost) -> void {
     if (cost >= best_cost) return;
@@ -63,19 +69,21 @@ bool factor(int n, int max_stages, std::vector<int> &best)
       best = cur;
       return;
     }
-    if ((int)cur.size() == max_stages) return;
+    if (cur.count == kMrStages) return;
     for (int R = from; R >= 2; --R)
       if (left % R == 0)
       {
-        cur.push_back(R);
+        cur.r[cur.count++] = R;
         self(self, left / R, R, cost + dft_cost(R) + kPassCost);
-        cur.pop_back();
+        --cur.count;
       }
   };
   rec(rec, n, 16, 0.f);
-  if (best.empty()) return false;
-  std::stable_sort(best.begin(), best.end(), [](int x, int y) { return (x & -x) > (y & -y); });
-  return true;
+  // insertion, equal shares in the order found
+  for (int i = 1; i < best.count; ++i)
+    for (int j = i; j > 0 && (best.r[j] & -best.r[j]) > (best.r[j - 1] & -best.r[j - 1]); --j)
+      std::swap(best.r[j], best.r[j - 1]);
+  return best.count > 0;
 }
 
 struct MrConfig { int C, threads; };
@@ -205,19 +213,19 @@ void mixed_free(MixedPlan *p)
 int mixed_create(long long n, MixedPlan **out, cudaStream_t st)
 {
   *out = nullptr;
-  std::vector<int> radix;
-  if (!mixed_length(n) || !factor((int)n, kMrStages, radix))
+  Radices radix;
+  if (!mixed_length(n) || !factor((int)n, radix))
     return set_error(FCB_ERR_UNSUPPORTED, "length %lld has no mixed-radix plan", n);
   MixedPlan *p = new (std::nothrow) MixedPlan;
   if (!p) return set_error(FCB_ERR_NOMEM, "mixed-radix plan");
   p->n = (int)n;
-  p->ns = (int)radix.size();
+  p->ns = radix.count;
   auto magic = [](int d) { return d == 1 ? 0u : (unsigned)(((1ULL << 32) + d - 1) / d); };
   int L = (int)n, tw = 0;
   for (int k = 0; k < p->ns; ++k)
   {
     MrStage &s = p->st[k];
-    s.R = radix[k];
+    s.R = radix.r[k];
     s.L = L;
     s.S = L / s.R;
     s.nb = (int)n / s.R;
@@ -230,7 +238,12 @@ int mixed_create(long long n, MixedPlan **out, cudaStream_t st)
   // block b of the last stage has the digits q1 .. q(ns-1), the first one the most significant;
   // its first output is q1 + R1 (q2 + R2 (q3 + ...))
   const int nb = p->st[p->ns - 1].nb;
-  std::vector<unsigned short> rev(nb);
+  const std::unique_ptr<unsigned short[]> rev(new (std::nothrow) unsigned short[nb]);
+  if (!rev)
+  {
+    mixed_free(p);
+    return set_error(FCB_ERR_NOMEM, "mixed-radix tables");
+  }
   for (int b = 0; b < nb; ++b)
   {
     int rest = b, j = 0;
@@ -261,7 +274,7 @@ int mixed_create(long long n, MixedPlan **out, cudaStream_t st)
     return set_error(FCB_ERR_NOMEM, "mixed-radix tables: %s", cudaGetErrorString(e));
   }
   // from pageable memory: the host buffer has been read when the call returns
-  e = cudaMemcpyAsync(p->rev, rev.data(), sizeof(unsigned short) * (size_t)nb, cudaMemcpyHostToDevice, st);
+  e = cudaMemcpyAsync(p->rev, rev.get(), sizeof(unsigned short) * (size_t)nb, cudaMemcpyHostToDevice, st);
   for (int k = 0; e == cudaSuccess && k + 1 < p->ns; ++k)
   {
     const long long m = (long long)(p->st[k].R / 2) * p->st[k].S;

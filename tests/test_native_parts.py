@@ -27,3 +27,8 @@ def _run(tmp_path, program, source):
 def test_bound_of_few_rows_is_stored_once_final(tmp_path):
     r = _run(tmp_path, "resident_bound", "fcb200.cu")
     assert r.returncode == 0, (r.returncode, r.stdout, r.stderr)
+
+
+def test_mixed_plans_report_failed_allocations(tmp_path):
+    r = _run(tmp_path, "mixed_alloc", "fcb_mixed.cu")
+    assert r.returncode == 0, (r.returncode, r.stdout, r.stderr)
