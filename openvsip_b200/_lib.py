@@ -8,6 +8,7 @@ from __future__ import annotations
 import ctypes
 import os
 import re
+import sys
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(HERE, "libfcb200.so")
@@ -120,6 +121,13 @@ def lib() -> ctypes.CDLL:
                 fn.argtypes = args
         _lib = L
     return _lib
+
+
+def torch_tag() -> str:
+    """The Python and the torch that the native call path (csrc/fcb_torch.cpp, which
+    inlines torch's accessors) has to be built for."""
+    import torch
+    return f"{sys.implementation.cache_tag} torch {torch.__version__}"
 
 
 def last_error() -> str:

@@ -81,23 +81,29 @@ def build(verbose: bool = False, force: bool = False) -> str:
 
 def build_torch(force: bool = False) -> str:
     """The native host path for CUDA tensors (csrc/fcb_torch.cpp), a Python
-    extension module against the installed torch."""
+    extension module against the installed torch: built again when that or the
+    Python changes (_fcb_torch.tag says what it was built for)."""
     import sysconfig
 
     import torch
+
+    from ._lib import torch_tag
     src = os.path.join(CSRC, "fcb_torch.cpp")
-    out = os.path.join(HERE, "_fcb_torch.so")
-    if not force and not _stale(out, [src]):
+    out, tag = os.path.join(HERE, "_fcb_torch.so"), os.path.join(HERE, "_fcb_torch.tag")
+    built_for = open(tag).read() if os.path.exists(tag) else ""
+    if not force and not _stale(out, [src]) and built_for == torch_tag():
         return out
     tdir = os.path.dirname(torch.__file__)
     cuda = os.path.dirname(os.path.dirname(os.path.realpath(nvcc())))
     cmd = [shutil.which("g++") or "g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
-           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", f'-DFCB_BUILT_FOR="{torch_tag()}"',
            f"-I{sysconfig.get_paths()['include']}", f"-I{tdir}/include", f"-I{tdir}/include/torch/csrc/api/include",
            f"-I{cuda}/include", src, "-o", out, f"-L{tdir}/lib", "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError(f"g++ failed: {' '.join(cmd)}\n{r.stdout}\n{r.stderr}")
+    with open(tag, "w") as f:
+        f.write(torch_tag())
     return out
 
 

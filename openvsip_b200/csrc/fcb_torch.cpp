@@ -108,4 +108,10 @@ PyModuleDef g_module = {PyModuleDef_HEAD_INIT, "_fcb_torch", nullptr, -1, g_meth
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__fcb_torch(void) { return PyModule_Create(&g_module); }
+// built_for: the Python and torch this was compiled against, whose object layouts it relies on
+PyMODINIT_FUNC PyInit__fcb_torch(void)
+{
+  PyObject *m = PyModule_Create(&g_module);
+  if (m && PyModule_AddStringConstant(m, "built_for", FCB_BUILT_FOR) < 0) Py_CLEAR(m);
+  return m;
+}

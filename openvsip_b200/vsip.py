@@ -172,8 +172,8 @@ def _put_transposed(out, yt):
 
 def _load_native(*args):
     """Stands for the native call path (csrc/fcb_torch.cpp) until the first call
-    on a tensor: loads it and makes that call.  Without the module every call
-    takes the ctypes path."""
+    on a tensor: loads it and makes that call.  Without the module, or with one
+    built for another torch or Python, every call takes the ctypes path."""
     global _native
     import sys
     if "torch" not in sys.modules:
@@ -181,6 +181,8 @@ def _load_native(*args):
     try:
         from . import _fcb_torch
     except ImportError:
+        _fcb_torch = None
+    if getattr(_fcb_torch, "built_for", None) != _lib.torch_tag():
         _native = _no_native
     else:
         L = lib()
