@@ -193,21 +193,24 @@ __global__ void dft_fp64_kernel(const float2 *in, const double2 *w, unsigned n, 
 
 // out[r][c] = v[c] m[r][c].  A thread keeps its columns' multipliers in registers and
 // goes down the rows, so an element costs its own load and store and nothing else
-// (HBM-bound: 16 bytes a sample; with a grid-stride loop over elements and its 64-bit
-// division, 1024 x 8192 took 32.8 us against 19.5, 4096 x 1000 18.4 against 7.0).  VEC: two columns a thread in 16-byte accesses,
-// for rows that all start 16-byte aligned.
-template <bool VEC>
+// (HBM-bound: 2^26 samples, 1.07 GB, take 163 us, 6.6 TB/s; a grid-stride loop over
+// elements with its 64-bit division took 210).  VEC: two columns a thread in 16-byte
+// accesses, for rows that all start 16-byte aligned.  DEEP: a CTA's threads also lie down
+// the rows (threadIdx.y), for matrices too narrow to fill it otherwise (the same samples in
+// 1, 4, 16 and 64 columns: 163 us against 2076, 712, 262 and 169 with a row at a time).
+template <bool VEC, bool DEEP>
 __global__ void __launch_bounds__(256) vmmul_kernel(const float2 *v, const float2 *m, long long m_rs, float2 *out,
                                                     long long out_rs, long long rows, long long cols)
 {
   begin_after_previous();
   const long long c = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * (VEC ? 2 : 1);
   if (c >= cols) return;
-  const long long step = gridDim.y;
+  const long long r0 = DEEP ? blockIdx.y * blockDim.y + threadIdx.y : blockIdx.y;
+  const long long step = DEEP ? gridDim.y * blockDim.y : gridDim.y;
   using V = std::conditional_t<VEC, float4, float2>;
   const float2 w0 = v[c], w1 = VEC ? v[c + 1] : w0;
   constexpr int B = 4;  // rows in flight (loads first: out may be m, so the compiler keeps the order)
-  for (long long r = blockIdx.y; r < rows; r += B * step)
+  for (long long r = r0; r < rows; r += B * step)
   {
     V b[B];
 #pragma unroll
@@ -440,12 +443,12 @@ int launch_rows(const KernelInfo *k, long long rows, const RowArgs &args, cudaSt
                        k->overlapped);
 }
 
-int launch_kernel(const void *fn, dim3 grid, int threads, int cluster, size_t smem, void **params, cudaStream_t st,
+int launch_kernel(const void *fn, dim3 grid, dim3 threads, int cluster, size_t smem, void **params, cudaStream_t st,
                   const char *what, bool overlapped)
 {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
-  cfg.blockDim = dim3(threads);
+  cfg.blockDim = threads;
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cudaLaunchAttribute attr[2];
@@ -533,14 +536,18 @@ int launch_vmmul(const float2 *v, const float2 *m, long long m_rs, float2 *out, 
   if (rows <= 0 || cols <= 0) return FCB_OK;
   auto even = [](const float2 *p, long long rs) { return reinterpret_cast<uintptr_t>(p) % 16 == 0 && rs % 2 == 0; };
   const bool vec = cols % 2 == 0 && even(m, m_rs) && even(out, out_rs);
-  const long long gx = (cols / (vec ? 2 : 1) + 255) / 256;
+  const long long across = cols / (vec ? 2 : 1), gx = (across + 255) / 256;
   if (gx > 0x7fffffffLL) return set_error(FCB_ERR_INVALID, "too many columns in one call");
+  // rows side by side in a CTA where at least two of them fit (see vmmul_kernel)
+  const int deep = across <= 128 ? 256 / (int)across : 1, lanes = deep > 1 ? (int)across : 256;
+  const long long groups = (rows + deep - 1) / deep;
   // eight CTAs for every SM, at most sixteen rows a thread
-  const long long gy = std::min<long long>(65535, std::max<long long>(std::min<long long>(rows, (148 * 8 + gx - 1) / gx),
-                                                                      rows / 16));
+  const long long gy = std::min<long long>(65535, std::max<long long>(std::min<long long>(groups, (148 * 8 + gx - 1) / gx),
+                                                                      groups / 16));
   void *params[] = {&v, &m, &m_rs, &out, &out_rs, &rows, &cols};
-  return launch_kernel(vec ? (const void *)&vmmul_kernel<true> : (const void *)&vmmul_kernel<false>,
-                       dim3((unsigned)gx, (unsigned)gy), 256, 1, 0, params, st, "vmmul launch");
+  const void *fn = deep > 1 ? (vec ? (const void *)&vmmul_kernel<true, true> : (const void *)&vmmul_kernel<false, true>)
+                            : (vec ? (const void *)&vmmul_kernel<true, false> : (const void *)&vmmul_kernel<false, false>);
+  return launch_kernel(fn, dim3((unsigned)gx, (unsigned)gy), dim3(lanes, deep), 1, 0, params, st, "vmmul launch");
 }
 
 int launch_transpose(const float2 *in, long long in_rs, float2 *out, long long out_rs, long long rows,

@@ -92,7 +92,7 @@ int prepare_kernel(const KernelInfo *k);
 // Launches a kernel in clusters of `cluster` CTAs; one that starts with
 // begin_after_previous() (overlapped) so that its launch overlaps the end of the
 // kernel before it in the stream.
-int launch_kernel(const void *fn, dim3 grid, int threads, int cluster, size_t smem, void **params, cudaStream_t st,
+int launch_kernel(const void *fn, dim3 grid, dim3 threads, int cluster, size_t smem, void **params, cudaStream_t st,
                   const char *what, bool overlapped = true);
 int launch_rows(const KernelInfo *k, long long rows, const RowArgs &args, cudaStream_t st);
 
