@@ -3,8 +3,9 @@
 // sizes, ctypes conversions) took 3 of the 6.3 us that a small call cost.
 //
 //   exec(kind, handle, in, out, n_in, n_out) -> status, or None
+//   vmmul(v, m, out) -> status, or None
 //
-// None means that the tensors are not two plain matrices (or do not match the
+// None means that the tensors are not plain matrices (or do not match the
 // plan): the caller then takes the general path, which converts what it can and
 // reports what it cannot.  Nothing is kept between calls.
 #include <Python.h>
@@ -16,6 +17,7 @@ namespace {
 
 using ExecFn = int (*)(void *, const void *, long long, void *, long long, long long, int);
 using StreamFn = int (*)(void *, void *);
+using VmmulFn = int (*)(const void *, const void *, long long, void *, long long, long long, long long, void *);
 
 // complex rows, real rows to half spectra and back, complex columns
 enum Kind { kRows = 0, kR2C = 1, kC2R = 2, kCols = 3, kKinds = 4 };
@@ -23,6 +25,7 @@ constexpr int kDevice = 1;  // FCB_DEVICE
 
 ExecFn g_exec[kKinds] = {};
 StreamFn g_set_stream = nullptr;
+VmmulFn g_vmmul = nullptr;
 
 struct Matrix
 {
@@ -30,22 +33,38 @@ struct Matrix
   long long rows = 0, cols = 0, rs = 0;
 };
 
-// A CUDA matrix of its own storage with unit-stride rows that do not overlap and
-// no lazy conjugate or negation.
-bool plain(PyObject *o, bool real, bool written, Matrix &m)
+// A CUDA tensor of its own storage whose memory holds its values (no lazy conjugate or
+// negation).
+bool held(PyObject *o, bool real)
 {
   if (!THPVariable_CheckExact(o)) return false;
   const at::Tensor &t = THPVariable_Unpack(o);
-  if (!t.is_cuda() || t.layout() != at::kStrided || t.dim() != 2 || !t.has_storage()) return false;
-  if (t.scalar_type() != (real ? at::kFloat : at::kComplexFloat) || t.is_conj() || t.is_neg()) return false;
-  if (written && t.requires_grad()) return false;
-  m.rows = t.size(0);
-  m.cols = t.size(1);
-  if (m.rows < 1 || m.cols < 1 || t.stride(1) != 1) return false;
+  return t.is_cuda() && t.layout() == at::kStrided && t.has_storage() &&
+         t.scalar_type() == (real ? at::kFloat : at::kComplexFloat) && !t.is_conj() && !t.is_neg();
+}
+
+// A matrix with unit-stride rows that do not overlap, or a vector: one row.
+bool plain(PyObject *o, bool real, Matrix &m)
+{
+  if (!held(o, real)) return false;
+  const at::Tensor &t = THPVariable_Unpack(o);
+  const int64_t d = t.dim();
+  if (d < 1 || d > 2) return false;
+  m.rows = d == 2 ? t.size(0) : 1;
+  m.cols = t.size(d - 1);
+  if (m.rows < 1 || m.cols < 1 || t.stride(d - 1) != 1) return false;
   m.rs = m.rows > 1 ? t.stride(0) : m.cols;
   if (m.rs < m.cols) return false;
   m.p = t.data_ptr();
   return true;
+}
+
+// What a column transform's transposing form refuses: a vector, an output that torch
+// must not write behind autograd's back.
+bool column_form(PyObject *in, PyObject *out)
+{
+  const at::Tensor &t = THPVariable_Unpack(out);
+  return THPVariable_Unpack(in).dim() == 2 && t.dim() == 2 && !t.requires_grad();
 }
 
 bool same_or_apart(const Matrix &a, const Matrix &b)
@@ -67,10 +86,11 @@ PyObject *exec(PyObject *, PyObject *const *args, Py_ssize_t nargs)
   void *stream = nullptr;
   try
   {
-    if (!plain(args[2], kind == kR2C, false, in) || !plain(args[3], kind == kC2R, true, out)) Py_RETURN_NONE;
+    if (!plain(args[2], kind == kR2C, in) || !plain(args[3], kind == kC2R, out)) Py_RETURN_NONE;
     if (in.rows != out.rows) Py_RETURN_NONE;
     if (kind == kCols)
     {
+      if (!column_form(args[2], args[3])) Py_RETURN_NONE;
       // a column plan: n_in the length, n_out the most columns
       if (in.rows != n_in || in.cols > n_out || in.cols != out.cols || !same_or_apart(in, out)) Py_RETURN_NONE;
     }
@@ -90,18 +110,46 @@ PyObject *exec(PyObject *, PyObject *const *args, Py_ssize_t nargs)
   return PyLong_FromLong(rc);
 }
 
-// bind(fcb_set_stream, fcb_exec, fcb_exec_r2c, fcb_exec_c2r, fcb_exec_cols): addresses
+// out[r][c] = v[c] m[r][c]
+PyObject *vmmul(PyObject *, PyObject *const *args, Py_ssize_t nargs)
+{
+  if (nargs != 3) return PyErr_Format(PyExc_TypeError, "vmmul takes three arguments");
+  Matrix m, out;
+  const void *v = nullptr;
+  void *stream = nullptr;
+  try
+  {
+    if (!g_vmmul || !held(args[0], false) || !plain(args[1], false, m) || !plain(args[2], false, out)) Py_RETURN_NONE;
+    const at::Tensor &t = THPVariable_Unpack(args[0]);
+    if (!t.is_contiguous() || t.numel() != m.cols || out.rows != m.rows || out.cols != m.cols) Py_RETURN_NONE;
+    v = t.data_ptr();
+    stream = c10::cuda::getCurrentCUDAStream().stream();
+  }
+  catch (...)
+  {
+    Py_RETURN_NONE;
+  }
+  int rc;
+  Py_BEGIN_ALLOW_THREADS
+  rc = g_vmmul(v, m.p, m.rs, out.p, out.rs, m.rows, m.cols, stream);
+  Py_END_ALLOW_THREADS
+  return PyLong_FromLong(rc);
+}
+
+// bind(fcb_set_stream, fcb_exec, fcb_exec_r2c, fcb_exec_c2r, fcb_exec_cols, fcb_vmmul_rows): addresses
 PyObject *bind(PyObject *, PyObject *const *args, Py_ssize_t nargs)
 {
-  if (nargs != 1 + kKinds) return PyErr_Format(PyExc_TypeError, "bind takes five addresses");
+  if (nargs != 2 + kKinds) return PyErr_Format(PyExc_TypeError, "bind takes six addresses");
   g_set_stream = reinterpret_cast<StreamFn>(PyLong_AsVoidPtr(args[0]));
   for (int i = 0; i < kKinds; ++i) g_exec[i] = reinterpret_cast<ExecFn>(PyLong_AsVoidPtr(args[1 + i]));
+  g_vmmul = reinterpret_cast<VmmulFn>(PyLong_AsVoidPtr(args[1 + kKinds]));
   if (PyErr_Occurred()) return nullptr;
   Py_RETURN_NONE;
 }
 
 PyMethodDef g_methods[] = {
     {"exec", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(exec)), METH_FASTCALL, nullptr},
+    {"vmmul", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(vmmul)), METH_FASTCALL, nullptr},
     {"bind", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(bind)), METH_FASTCALL, nullptr},
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef g_module = {PyModuleDef_HEAD_INIT, "_fcb_torch", nullptr, -1, g_methods, nullptr, nullptr, nullptr, nullptr};

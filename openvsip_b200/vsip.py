@@ -170,26 +170,35 @@ def _put_transposed(out, yt):
     return out
 
 
-def _load_native(*args):
-    """Stands for the native call path (csrc/fcb_torch.cpp) until the first call
-    on a tensor: loads it and makes that call.  Without the module, or with one
-    built for another torch or Python, every call takes the ctypes path."""
-    global _native
+def _load() -> bool:
+    """Loads the native call path (csrc/fcb_torch.cpp) if torch is there.  Without
+    the module, or with one built for another torch or Python, every call takes
+    the ctypes path."""
+    global _native, _native_vmmul
     import sys
     if "torch" not in sys.modules:
-        return None
+        return False
     try:
         from . import _fcb_torch
     except ImportError:
         _fcb_torch = None
     if getattr(_fcb_torch, "built_for", None) != _lib.torch_tag():
-        _native = _no_native
+        _native = _native_vmmul = _no_native
     else:
         L = lib()
         _fcb_torch.bind(*(ctypes.cast(f, ctypes.c_void_p).value for f in (
-            L.fcb_set_stream, L.fcb_exec, L.fcb_exec_r2c, L.fcb_exec_c2r, L.fcb_exec_cols)))
-        _native = _fcb_torch.exec
-    return _native(*args)
+            L.fcb_set_stream, L.fcb_exec, L.fcb_exec_r2c, L.fcb_exec_c2r, L.fcb_exec_cols, L.fcb_vmmul_rows)))
+        _native, _native_vmmul = _fcb_torch.exec, _fcb_torch.vmmul
+    return True
+
+
+def _load_native(*args):
+    """Stands for the native calls until the first one on a tensor."""
+    return _native(*args) if _load() else None
+
+
+def _load_vmmul(*args):
+    return _native_vmmul(*args) if _load() else None
 
 
 def _no_native(*args):
@@ -197,6 +206,7 @@ def _no_native(*args):
 
 
 _native = _load_native  # (kind, plan, in, out, n_in, n_out) -> status, or None: not plain CUDA matrices
+_native_vmmul = _load_vmmul  # (v, m, out) -> status, or None
 _ROWS, _R2C, _C2R, _COLS = range(4)
 
 
@@ -486,11 +496,14 @@ def vmmul(v, m, out=None):
 
     v and m must be CUDA complex64 tensors (device data); the op is queued on
     the current torch stream."""
-    import torch
     if not (_is_torch(v) and _is_torch(m) and v.is_cuda and m.is_cuda):
         raise TypeError("vmmul runs on the GPU: pass CUDA complex64 tensors")
     if out is None:
-        out = torch.empty_like(m)
+        out = _torch_mod().empty_like(m)
+    rc = _native_vmmul(v, m, out)
+    if rc is not None:
+        check(rc)
+        return out
     mp, r, c, mrs, _ = _desc(m, False)
     op, r2, c2, ors, _ = _desc(out, True)
     v = _held(v).contiguous()
