@@ -185,7 +185,9 @@ FCB_API int fcb_exec_async(fcb_plan plan, const fcb_cf32 *in, long long in_rs, f
 
 /* Column transforms without transposing: an n x cols matrix (row strides in_rs /
  * out_rs >= cols), each of its columns transformed; in place with equal strides
- * is allowed.  A host call returns with the output written.  Replaces fftm_backend<..., 1, D>
+ * is allowed.  A host call returns with the output written (in blocks of columns through the
+ * plan's staging buffers and, where pageable, the shared pinned ones: one such call at a time).
+ * Replaces fftm_backend<..., 1, D>
  * over columns (src/ovxx/fftw/fftw.cpp:904-977).  fcb_supported_cols says
  * which n have such a kernel; fcb_plan_fftm_cols makes a plan that serves
  * fcb_exec_cols (up to cols_max columns) and, over rows of n, fcb_exec. */

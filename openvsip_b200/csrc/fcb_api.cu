@@ -77,9 +77,6 @@ struct fcb_plan_s
   // any such length: the mixed-radix kernel.
   MixedPlan *mx = nullptr;
   float2 *mx_rep = nullptr;                    // fastconv: replica table(s), last-stage order
-  std::mutex cols_mu;                          // host column calls: one at a time has the block below
-  float2 *cstage = nullptr;                    // device copy of a block of columns
-  long long cstage_cols = 0;
   // Real-input rows of n = rn samples: 1 = real -> complex (n/2 + 1 outputs),
   // 2 = complex -> real.  Even n: a length-n/2 complex plan plus the split /
   // merge step; odd n: a length-n complex plan on expanded rows.
@@ -189,7 +186,6 @@ void plan_free(fcb_plan p)
   mixed_free(p->mxc);
   cudaFree(p->twx);
   cudaFree(p->mx_rep);
-  cudaFree(p->cstage);
   plan_free(p->cplx);
   cudaFree(p->rtw);
   cudaFree(p->rtw4);
@@ -853,7 +849,7 @@ int ensure_staging(fcb_plan p, long long chunk_rows, int depth)
 // stays busy in both directions; a buffer is refilled once its copy out is done.
 // sync = false (fcb_exec_async): return once everything is queued.
 int exec_host_staged(fcb_plan p, const float2 *in, long long in_rs, float2 *out, long long out_rs,
-                     long long rows, bool stage_in, bool stage_out);
+                     long long rows, bool stage_in, bool stage_out, bool columns = false);
 
 int exec_host(fcb_plan p, const float2 *in, long long in_rs, float2 *out, long long out_rs,
               long long rows, bool sync = true)
@@ -962,77 +958,84 @@ int exec_host(fcb_plan p, const float2 *in, long long in_rs, float2 *out, long l
 // engines and the kernels work on the neighbouring chunks.  A pinned side
 // moves directly.  Returns when the output is written, queued or not;
 // kNoPinned, before any work, if the pinned buffers could not be had.
+// With `columns`, `count` columns of length n instead of rows: a chunk is a block of
+// adjacent ones, n short rows on the host and packed on the device.
 int exec_host_staged(fcb_plan p, const float2 *in, long long in_rs, float2 *out, long long out_rs,
-                     long long rows, bool stage_in, bool stage_out)
+                     long long count, bool stage_in, bool stage_out, bool columns)
 {
   std::lock_guard<std::mutex> lk(pinned().mu);
-  const size_t row_bytes = sizeof(float2) * (size_t)p->n;
-  long long chunk = std::max<long long>(1, stage_bytes() / (long long)row_bytes);
+  const size_t one = sizeof(float2) * (size_t)p->n;  // a row or a column
+  long long chunk = std::max<long long>(1, stage_bytes() / (long long)one);
   long long alloc = 2 * chunk;  // the device buffers as the pinned path sizes them
-  if (p->k && p->k->cluster == 1)
+  if (!columns && p->k && p->k->cluster == 1)
   {
     chunk = std::max<long long>(chunk, p->k->rows_per_cta);
     alloc = std::max<long long>(alloc, p->k->rows_per_cta);
   }
-  chunk = std::min(chunk, rows);
+  chunk = std::min(chunk, count);
   const int depth = stage_depth();
-  int rc = ensure_staging(p, std::min(alloc, rows), depth);
+  int rc = ensure_staging(p, std::min(alloc, count), depth);
   if (rc) return rc;
-  if (stage_in && (rc = ensure_host_staging(p, 0, row_bytes * (size_t)chunk, depth))) return rc;
-  if (stage_out && (rc = ensure_host_staging(p, 1, row_bytes * (size_t)chunk, depth))) return rc;
+  if (stage_in && (rc = ensure_host_staging(p, 0, one * (size_t)chunk, depth))) return rc;
+  if (stage_out && (rc = ensure_host_staging(p, 1, one * (size_t)chunk, depth))) return rc;
   cudaEventRecord(p->ev_start, p->stream);
   cudaStreamWaitEvent(p->cin, p->ev_start, 0);
   cudaStreamWaitEvent(p->cout, p->ev_start, 0);
-  const long long nc = (rows + chunk - 1) / chunk;
+  const long long nc = (count + chunk - 1) / chunk;
   const int b0 = p->stage_next % depth;
   p->stage_next = (int)((b0 + nc) % depth);
   const int lag = depth - 1;  // chunks between a chunk's copy in and its copy out on the host
   auto buf_of = [&](long long c) { return (int)((b0 + c) % depth); };
+  // chunk c on the host: `rows` rows of rb bytes, from element `at`
+  struct Block { long long k; size_t rb, rows; };
+  auto block = [&](long long c) -> Block {
+    const long long k = std::min(chunk, count - c * chunk);
+    return columns ? Block{k, sizeof(float2) * (size_t)k, (size_t)p->n} : Block{k, one, (size_t)k};
+  };
+  auto at = [&](long long c, long long rs) { return columns ? c * chunk : c * chunk * rs; };
+  auto copy = [](void *dst, size_t dp, const void *src, size_t sp, const Block &k, cudaMemcpyKind kind, cudaStream_t st) {
+    return dp == k.rb && sp == k.rb ? cudaMemcpyAsync(dst, src, k.rb * k.rows, kind, st)
+                                    : cudaMemcpy2DAsync(dst, dp, src, sp, k.rb, k.rows, kind, st);
+  };
   // copy chunk d's result from its pinned buffer to the caller's rows
   auto drain = [&](long long d) -> int {
     const int b = buf_of(d);
-    const long long r0 = d * chunk, nr = std::min(chunk, rows - r0);
+    const Block k = block(d);
     const cudaError_t e = cudaEventSynchronize(p->ev_h[1][b]);
     if (e != cudaSuccess) return cuda_error(e, "device->host copy");
-    host_copy_rows(out + r0 * out_rs, sizeof(float2) * (size_t)out_rs, pinned().buf[1][b], row_bytes, row_bytes,
-                   (size_t)nr);
+    host_copy_rows(out + at(d, out_rs), sizeof(float2) * (size_t)out_rs, pinned().buf[1][b], k.rb, k.rb, k.rows);
     return FCB_OK;
   };
   for (long long c = 0; c < nc; ++c)
   {
     const int b = buf_of(c);
-    const long long r0 = c * chunk, nr = std::min(chunk, rows - r0);
-    const float2 *src = in + r0 * in_rs;
-    long long src_rs = in_rs;
+    const Block k = block(c);
+    const float2 *src = in + at(c, in_rs);
+    size_t src_pitch = sizeof(float2) * (size_t)in_rs;
     if (stage_in)
     {
       // the pinned buffer's previous chunk has moved in
       cudaError_t e = cudaEventSynchronize(p->ev_h[0][b]);
       if (e != cudaSuccess) return host_done(p, cuda_error(e, "host->device copy"), "fcb_exec (host)");
-      host_copy_rows(pinned().buf[0][b], row_bytes, src, sizeof(float2) * (size_t)in_rs, row_bytes, (size_t)nr);
+      host_copy_rows(pinned().buf[0][b], k.rb, src, src_pitch, k.rb, k.rows);
       src = pinned().buf[0][b];
-      src_rs = p->n;
+      src_pitch = k.rb;
     }
     float2 *buf = p->stage[b];
     cudaStreamWaitEvent(p->cin, p->ev_out[b], 0);
-    cudaError_t e = src_rs == p->n
-                      ? cudaMemcpyAsync(buf, src, row_bytes * (size_t)nr, cudaMemcpyHostToDevice, p->cin)
-                      : cudaMemcpy2DAsync(buf, row_bytes, src, sizeof(float2) * (size_t)src_rs, row_bytes, (size_t)nr,
-                                          cudaMemcpyHostToDevice, p->cin);
+    cudaError_t e = copy(buf, k.rb, src, src_pitch, k, cudaMemcpyHostToDevice, p->cin);
     if (e != cudaSuccess) return host_done(p, cuda_error(e, "host->device copy"), "fcb_exec (host)");
     cudaEventRecord(p->ev_in[b], p->cin);
     if (stage_in) cudaEventRecord(p->ev_h[0][b], p->cin);
     cudaStreamWaitEvent(p->stream, p->ev_in[b], 0);
-    rc = exec_device(p, buf, p->n, buf, p->n, nr, r0, p->stream, 0);
+    rc = columns ? mixed_transform(p->mx, true, buf, k.k, buf, k.k, k.k, p->mode == kInv, p->scale, p->stream)
+                 : exec_device(p, buf, p->n, buf, p->n, k.k, c * chunk, p->stream, 0);
     if (rc) return host_done(p, rc, "fcb_exec (host)");
     cudaEventRecord(p->ev_k[b], p->stream);
     cudaStreamWaitEvent(p->cout, p->ev_k[b], 0);
     // the output's pinned buffer was drained on the host depth chunks ago
-    e = stage_out ? cudaMemcpyAsync(pinned().buf[1][b], buf, row_bytes * (size_t)nr, cudaMemcpyDeviceToHost, p->cout)
-        : out_rs == p->n
-          ? cudaMemcpyAsync(out + r0 * out_rs, buf, row_bytes * (size_t)nr, cudaMemcpyDeviceToHost, p->cout)
-          : cudaMemcpy2DAsync(out + r0 * out_rs, sizeof(float2) * (size_t)out_rs, buf, row_bytes, row_bytes,
-                              (size_t)nr, cudaMemcpyDeviceToHost, p->cout);
+    e = stage_out ? copy(pinned().buf[1][b], k.rb, buf, k.rb, k, cudaMemcpyDeviceToHost, p->cout)
+                  : copy(out + at(c, out_rs), sizeof(float2) * (size_t)out_rs, buf, k.rb, k, cudaMemcpyDeviceToHost, p->cout);
     if (e != cudaSuccess) return host_done(p, cuda_error(e, "device->host copy"), "fcb_exec (host)");
     cudaEventRecord(p->ev_out[b], p->cout);
     if (stage_out) cudaEventRecord(p->ev_h[1][b], p->cout);
@@ -1049,6 +1052,25 @@ int exec_host_staged(fcb_plan p, const float2 *in, long long in_rs, float2 *out,
       if (rc) return host_done(p, rc, "fcb_exec (host)");
     }
   return host_done(p, FCB_OK, "fcb_exec (host)");
+}
+
+// Columns on host pointers.  A side is staged where it is pageable, and where the copy
+// engine would move many short rows, about 36 ns each (pinned strided arrays, 20 columns of
+// 2048 / 8000 / 14000: 233 / 766 / 1378 us moved as they are, 117 / 190 / 452 staged; but 20 of
+// 128 59 / 97, one of 8000 68 / 99, 100 of 8000 1028 / 834 with rows of 800 bytes).  Pageable
+// arrays, 20 columns of 2048 / 14000: 116 / 478 us, 1144 of 756 573 us (with whole-array copies
+// one after the other 369 / 1622 / 1259, by transposing on the host 190 / 1108 / 3136).
+int exec_cols_host(fcb_plan p, const float2 *in, long long in_rs, float2 *out, long long out_rs, long long cols)
+{
+  const long long n = p->n, chunk = std::min(cols, std::max<long long>(1, stage_bytes() / (8 * n)));
+  const bool short_rows = n >= 1000 && chunk > 1 && 8 * chunk < 512;
+  auto staged = [&](const float2 *x, long long rs) {
+    return (short_rows && rs != chunk) || host_pageable(x, sizeof(float2) * (size_t)((n - 1) * rs + cols));
+  };
+  const bool stage_in = staged(in, in_rs), stage_out = staged(out, out_rs);
+  const int rc = exec_host_staged(p, in, in_rs, out, out_rs, cols, stage_in, stage_out, true);
+  // no pinned memory to be had: the CUDA runtime copies the pageable memory
+  return rc == kNoPinned ? exec_host_staged(p, in, in_rs, out, out_rs, cols, false, false, true) : rc;
 }
 
 }  // namespace
@@ -1152,30 +1174,7 @@ int fcb_exec_cols(fcb_plan p, const fcb_cf32 *in, long long in_rs, fcb_cf32 *out
   float2 *o2 = reinterpret_cast<float2 *>(out);
   if (where == FCB_DEVICE)
     return mixed_transform(p->mx, true, i2, in_rs, o2, out_rs, cols, p->mode == kInv, p->scale, p->stream);
-  // host columns: blocks of them through one device buffer, which threads that share the plan
-  // take in turn (as they take the shared pinned buffers of the row calls)
-  std::lock_guard<std::mutex> turn(p->cols_mu);
-  const long long n = p->n, chunk = std::min(cols, std::max<long long>(1, (long long)(4 * stage_bytes()) / (8 * n)));
-  if (p->cstage_cols < chunk)
-  {
-    cudaFree(p->cstage);
-    p->cstage = nullptr;
-    p->cstage_cols = 0;
-    const cudaError_t e = cudaMalloc(&p->cstage, sizeof(float2) * (size_t)(chunk * n));
-    if (e != cudaSuccess) return set_error(FCB_ERR_NOMEM, "staging buffer: %s", cudaGetErrorString(e));
-    p->cstage_cols = chunk;
-  }
-  int rc = FCB_OK;
-  for (long long c0 = 0; !rc && c0 < cols; c0 += chunk)
-  {
-    const long long nc = std::min(chunk, cols - c0);
-    const size_t rb = sizeof(float2) * (size_t)nc;
-    rc = copy_h2d(p, p->cstage, rb, i2 + c0, sizeof(float2) * (size_t)in_rs, rb, (size_t)n, p->stream);
-    if (!rc)
-      rc = mixed_transform(p->mx, true, p->cstage, nc, p->cstage, nc, nc, p->mode == kInv, p->scale, p->stream);
-    if (!rc) rc = copy_d2h(p, o2 + c0, sizeof(float2) * (size_t)out_rs, p->cstage, rb, rb, (size_t)n, p->stream);
-  }
-  return host_done(p, rc, "fcb_exec_cols (host)");
+  return exec_cols_host(p, i2, in_rs, o2, out_rs, cols);
 }
 
 int fcb_plan_fastconv(long long n, long long rows_max, const fcb_cf32 *replica, long long replica_rows,
