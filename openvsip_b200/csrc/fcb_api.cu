@@ -232,8 +232,9 @@ int plan_common(fcb_plan p, long long n, long long rows_max, int mode)
 // length up to the longest row that fits shared memory.  Against Bluestein's
 // algorithm (two transforms of at least twice the length) it measured 1.3 to 6.7
 // times faster for transforms and 1.5 to 8.5 times for the fast convolution, at
-// 1 to 100000 rows of 18 to 28561 samples; powers of two stay with the row
-// kernels, which are as fast at 1024 and keep two samples per instruction.
+// 1 to 100000 rows of 18 to 28561 samples (but see blue_is_faster); powers of two
+// stay with the row kernels, which are as fast at 1024 and keep two samples per
+// instruction.
 int mixed_setup(fcb_plan p, long long n, long long rows_max, int mode)
 {
   int rc = check_device();
@@ -248,6 +249,16 @@ int mixed_setup(fcb_plan p, long long n, long long rows_max, int mode)
   p->stream = p->own_stream;
   return mixed_create(n, &p->mx, p->stream);
 }
+
+// Transforms of mixed-radix lengths that stay with Bluestein's algorithm: plans for few
+// long rows, where its clusters spread a row over more SMs, of lengths whose last
+// mixed-radix stage reads its blocks 16-way bank-conflicted (multiples of 256).  1 and 30
+// rows of 25344 / 26880 / 28672 samples: mixed 31.9 and 32.5, 32.4 and 33.4, 33.9 and 34.5
+// us, Bluestein 16.9 and 30.8, 17.1 and 30.9, 17.3 and 31.2; 25088: 31.0 and 29.8 for 19
+// rows; other lengths near 28000: 20 to 33 and 30.  33 clusters fit; from 34 rows they take a second
+// turn: 58 against 33 us.  By the plan's count, so that a row's result does not depend on
+// how many a call passes.
+bool blue_is_faster(long long n, long long rows_max) { return n > 25088 && n % 256 == 0 && rows_max <= 33; }
 
 // Bluestein plan for non-power-of-two n: a chirp and an inner length-m
 // fastconv plan per direction needed (fwd / inv), and one work buffer.
@@ -1113,7 +1124,7 @@ int fcb_plan_fftm(long long n, long long rows_max, int exponent, float scale, fc
   if (!p) return set_error(FCB_ERR_NOMEM, "plan allocation");
   p->scale = scale;
   const int mode = exponent == FCB_FORWARD ? kFwd : kInv;
-  const bool mixed = blue_length(n) && mixed_length(n), blue = blue_length(n) && !mixed;
+  const bool mixed = blue_length(n) && mixed_length(n) && !blue_is_faster(n, rows_max), blue = blue_length(n) && !mixed;
   int rc = mixed ? mixed_setup(p, n, rows_max, mode)
          : blue ? blue_setup(p, n, rows_max, mode, mode == kFwd, mode == kInv)
                 : plan_common(p, n, rows_max, mode);
