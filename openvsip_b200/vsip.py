@@ -328,17 +328,17 @@ class Fftm(_Plan):
         self.exponent = _exponent(direction)
         self.scale = float(scale)
         n, count = (self.cols, self.rows) if self.axis == row else (self.rows, self.cols)
-        h = ctypes.c_void_p()
-        plan = lib().fcb_plan_fftm if self.axis == row else lib().fcb_plan_fftm_cols
-        check(plan(n, count, self.exponent, self.scale, ctypes.byref(h)))
-        self._handle = h
-        self._n = n
         # Few columns of a long power of two are quicker as rows (the row kernel spreads a row
         # over more threads): 64 of 4096 9.7 us against 11.9, 64 of 8192 13.9 against 21.3; 128 of
         # 4096 the same, 256 of 4096 18.8 against 12.4, of 8192 33 against 22.6.  By the plan's
         # count, so that a column's result does not depend on how many a call passes.
         few = n >= 4096 and n & (n - 1) == 0 and count <= 128
         self._col_kernel = self.axis == col and not few and bool(lib().fcb_supported_cols(n))
+        h = ctypes.c_void_p()
+        plan = lib().fcb_plan_fftm_cols if self._col_kernel else lib().fcb_plan_fftm
+        check(plan(n, count, self.exponent, self.scale, ctypes.byref(h)))
+        self._handle = h
+        self._n = n
 
     def __call__(self, inp, out=None):
         """By reference: ``fftm(in, out)``; ``fftm(in)`` returns a new result (by value)."""
