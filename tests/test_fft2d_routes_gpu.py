@@ -1,5 +1,6 @@
 """2-D transforms by each of their routes against FP64: tall matrices of few columns
-(rows and transposes, or the column kernel)."""
+(rows and transposes, or the column kernel), the two transposing passes, columns that
+have no kernel of their own."""
 import numpy as np
 import pytest
 
@@ -10,7 +11,7 @@ pytestmark = pytest.mark.gpu
 RTOL = 2e-6
 
 
-def _check(oracle, rows, cols):
+def _check(rows, cols):
     """Forward and inverse, strided and in place, on the device and on the host."""
     import torch
     rng = np.random.default_rng(rows + 3 * cols)
@@ -33,8 +34,22 @@ def _check(oracle, rows, cols):
 
 @pytest.mark.parametrize("rows,cols", [(8192, 1), (8192, 7), (8192, 8), (8192, 16), (8192, 32), (8192, 100), (8192, 128),
                                        (8192, 129), (4096, 32), (4096, 1), (2048, 16), (16384, 32)])
-def test_tall_matrices(oracle, rows, cols):
-    _check(oracle, rows, cols)
+def test_tall_matrices(rows, cols):
+    _check(rows, cols)
+
+
+# two transposing passes: rows of 16384 (one a CTA), columns whose rest is too long for the
+# column kernel, and the sizes below those of the row pass that takes the columns along
+@pytest.mark.parametrize("rows,cols", [(128, 16384), (4096, 16384), (16384, 8192), (2048, 256), (2048, 64)])
+def test_transposing_passes(rows, cols):
+    _check(rows, cols)
+
+
+# columns of a length with a large prime factor, or too long: a row pass, a transpose,
+# a row pass and a transpose back; their transposed sizes take the column kernel
+@pytest.mark.parametrize("rows,cols", [(67, 100), (100, 67), (1007, 64), (1, 777), (16384, 100), (100, 16384), (17, 17)])
+def test_columns_without_a_kernel(rows, cols):
+    _check(rows, cols)
 
 
 def test_few_tall_columns_cost_no_more_than_rows_and_transposes():
