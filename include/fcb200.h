@@ -95,7 +95,8 @@ FCB_API int fcb_init(int device);
 /* 1 if n is a supported row length for Fftm and fast-convolution plans: any
  * length in [1, 32768], or a power of two up to 65536.  Powers of two run as
  * one fused pass, and so do lengths up to 28672 with no prime factor above 13
- * (mixed radix); other lengths by Bluestein's chirp-z algorithm: the fused
+ * (mixed radix; but for transforms of at most 33 rows of a multiple of 256
+ * above 25088); other lengths by Bluestein's chirp-z algorithm: the fused
  * kernel runs on work rows of the next power of two >= 2n - 1 samples and
  * applies the chirps, the zero padding and the truncation to n samples on its
  * own loads and stores (one pass per transform).  The reference's FFTW
@@ -117,8 +118,9 @@ FCB_API int fcb_plan_fftm(long long n, long long rows_max, int exponent, float s
  * fftm_backend<float, complex<float>, A, fft_fwd> and
  * fftm_backend<complex<float>, float, A, fft_inv> (src/ovxx/signal/fft/
  * backend.hpp:600-694; FFTW rows src/ovxx/fftw/fftw.cpp:778-903).  Even n:
- * one length-n/2 complex row FFT plus a split (forward) or merge (inverse)
- * pass; odd n: the length-n complex row FFT. */
+ * one length-n/2 complex row FFT and a split (forward) or merge (inverse),
+ * within the row kernel where n/2 is a power of two (the split up to 16384), as
+ * a pass of its own otherwise; odd n: the length-n complex row FFT. */
 FCB_API int fcb_supported_real_length(long long n);
 FCB_API int fcb_plan_fftm_real(long long n, long long rows_max, int exponent, float scale,
                                fcb_plan *plan);
@@ -135,11 +137,14 @@ FCB_API int fcb_exec_c2r(fcb_plan plan, const fcb_cf32 *in, long long in_rs, flo
  * takes rows == the plan's rows.  Replaces fft_backend<2, complex<float>,
  * complex<float>, S> (src/ovxx/signal/fft/backend.hpp:294-375; FFTW 2-D plan
  * src/ovxx/fftw/fftw.cpp:436-511), used by vsip::Fft<const_Matrix, ...>.
- * Both dimensions powers of two in [64, 16384]: two passes, each a row
- * transform that stores its result transposed (one rows x cols scratch
- * matrix).  Other dimensions (each any length fcb_supported_length accepts):
- * a row pass, a transpose, a column pass and a transpose back (two scratch
- * matrices). */
+ * Dimensions: each any length fcb_supported_length accepts.  Large powers of
+ * two: a row pass that takes the columns' first stage along, and the column
+ * kernel on the rest; smaller ones of up to 1024 rows, and rows of a length
+ * with a column kernel (fcb_supported_cols): a row pass and the column kernel;
+ * the remaining powers of two in [64, 16384]: two row passes that store
+ * transposed (one rows x cols scratch matrix).  Otherwise, and for 8 to
+ * 128 columns of 8192: a row pass, a transpose, a row pass and a transpose back
+ * (two scratch matrices). */
 FCB_API int fcb_plan_fft2d(long long rows, long long cols, int exponent, float scale,
                            fcb_plan *plan);
 

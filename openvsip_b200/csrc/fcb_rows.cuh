@@ -24,9 +24,11 @@ KernelInfo rows_info()
   k.rows_per_cta = S::ROWS;
   k.smem = S::SMEM;
   k.tw_bytes = S::tw_bytes();
-  // The kernel for calls of few rows (same tables, same arithmetic), for the variants that are
-  // the defaults: the FEW form of the same CTA up to 8192 samples; from 16384 up, where a CTA of
-  // 512 threads fills an SM anyway, twice as many CTAs of 256 threads for a row.
+  // The kernel for calls of few rows (same tables, same arithmetic), for the default variants of
+  // 32 samples a thread: the FEW form of the same CTA up to 8192 samples; from 16384 up, where a
+  // CTA of 512 threads fills an SM anyway, twice as many CTAs of 256 threads for a row.  The wide
+  // variant, the default of the fused convolution at 16384 and the transforms at 32768, has none:
+  // its tables and stages are others, and rows would come out differently.
   if constexpr (!FEW && EPTW == 32 && MODE != kCoefs)
   {
     constexpr bool same = (T == 128 && LOGN <= 12) || (T == 256 && (LOGN < kMin128 || LOGN == 13));
