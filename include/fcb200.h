@@ -95,8 +95,8 @@ FCB_API int fcb_init(int device);
 /* 1 if n is a supported row length for Fftm and fast-convolution plans: any
  * length in [1, 32768], or a power of two up to 65536.  Powers of two run as
  * one fused pass, and so do lengths up to 28672 with no prime factor above 13
- * (mixed radix; but for transforms of at most 33 rows of a multiple of 256
- * above 25088); other lengths by Bluestein's chirp-z algorithm: the fused
+ * (mixed radix; but for transforms planned for at most 33 rows of 28000 or a
+ * multiple of 256 above 25000); other lengths by Bluestein's chirp-z algorithm: the fused
  * kernel runs on work rows of the next power of two >= 2n - 1 samples and
  * applies the chirps, the zero padding and the truncation to n samples on its
  * own loads and stores (one pass per transform).  The reference's FFTW

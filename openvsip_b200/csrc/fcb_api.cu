@@ -252,13 +252,13 @@ int mixed_setup(fcb_plan p, long long n, long long rows_max, int mode)
 
 // Transforms of mixed-radix lengths that stay with Bluestein's algorithm: plans for few
 // long rows, where its clusters spread a row over more SMs, of lengths whose last
-// mixed-radix stage reads its blocks 16-way bank-conflicted (multiples of 256).  1 and 30
-// rows of 25344 / 26880 / 28672 samples: mixed 31.9 and 32.5, 32.4 and 33.4, 33.9 and 34.5
-// us, Bluestein 16.9 and 30.8, 17.1 and 30.9, 17.3 and 31.2; 25088: 31.0 and 29.8 for 19
-// rows; other lengths near 28000: 20 to 33 and 30.  33 clusters fit; from 34 rows they take a second
-// turn: 58 against 33 us.  By the plan's count, so that a row's result does not depend on
-// how many a call passes.
-bool blue_is_faster(long long n, long long rows_max) { return n > 25088 && n % 256 == 0 && rows_max <= 33; }
+// mixed-radix stage has bank conflicts (multiples of 256, and 28000).  1 and 30 rows of
+// 25344 / 26880 / 28672 samples: mixed 31.9 and 32.5, 32.4 and 33.4, 33.9 and 34.5 us,
+// Bluestein 16.9 and 30.8, 17.1 and 30.9, 17.3 and 31.2; 24576: 29.8 and 29.7 for 19 rows;
+// other lengths near 28000: 20 to 29 and 30.  33 clusters fit; from 34 rows they take a
+// second turn: 58 against 33 us.  By the plan's count, so that a row's result does not
+// depend on how many a call passes.
+bool blue_is_faster(long long n, long long rows_max) { return rows_max <= 33 && n > 25000 && mixed_conflicts(n); }
 
 // Bluestein plan for non-power-of-two n: a chirp and an inner length-m
 // fastconv plan per direction needed (fwd / inv), and one work buffer.

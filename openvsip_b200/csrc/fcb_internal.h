@@ -120,6 +120,7 @@ int scale_copy(const float2 *in, float2 *out, long long total, float s, cudaStre
 struct MixedPlan;
 bool mixed_length(long long n);
 bool mixed_columns(long long n);  // lengths whose columns mixed_transform takes
+bool mixed_conflicts(long long n);  // adjacent blocks of a row's last stage share a bank
 int mixed_create(long long n, MixedPlan **out, cudaStream_t st);
 void mixed_free(MixedPlan *p);
 void mixed_info(const MixedPlan *p, long long rows, int *rows_per_cta, int *smem, int *threads);

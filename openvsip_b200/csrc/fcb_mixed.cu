@@ -202,6 +202,14 @@ bool mixed_length(long long n)
   return n == 1;
 }
 
+// The last stage of a row takes its blocks in output order: those of adjacent threads lie n / (first radix) samples
+// apart, and where that is a multiple of 16 (128 bytes) as many of a half-warp's threads as the radix read the same bank.
+bool mixed_conflicts(long long n)
+{
+  Radices radix;
+  return mixed_length(n) && factor((int)n, radix) && radix.r[0] >= 14 && n / radix.r[0] % 16 == 0;
+}
+
 void mixed_free(MixedPlan *p)
 {
   if (!p) return;

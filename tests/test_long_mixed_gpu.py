@@ -1,5 +1,5 @@
-"""Few long rows of lengths that are multiples of 256 (7 * 4096, 13 * 2048, ..): plans for
-up to 33 rows, and for more, on both sides of the change of algorithm."""
+"""Few long rows of lengths whose last mixed-radix stage has bank conflicts (multiples of 256,
+28000): plans for up to 33 rows, and for more, on both sides of the change of algorithm."""
 import numpy as np
 import pytest
 
@@ -10,7 +10,7 @@ pytestmark = pytest.mark.gpu
 RTOL = 2e-6
 
 
-@pytest.mark.parametrize("n", [25088, 25344, 28672])
+@pytest.mark.parametrize("n", [24576, 25088, 28000, 28672])
 @pytest.mark.parametrize("rows", [1, 33, 34])
 def test_vs_fp64(oracle, n, rows):
     x = crandn(np.random.default_rng(n + rows), (rows, n))
@@ -24,7 +24,7 @@ def test_vs_fp64(oracle, n, rows):
     assert oracle.rel_l2(FftmReal(rows, 2 * n, fft_inv, 0.5 / n)(half.astype(np.complex64)), r) <= RTOL
 
 
-@pytest.mark.parametrize("n", [26880, 28672])
+@pytest.mark.parametrize("n", [26880, 28000, 28672])
 def test_few_planned_rows_are_spread_over_the_gpu(n):
     import torch
     x = torch.ones(8, n, dtype=torch.complex64, device="cuda")
