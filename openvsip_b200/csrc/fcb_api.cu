@@ -990,10 +990,16 @@ int exec_host_staged(fcb_plan p, const float2 *in, long long in_rs, float2 *out,
   if (rc) return rc;
   if (stage_in && (rc = ensure_host_staging(p, 0, one * (size_t)chunk, depth))) return rc;
   if (stage_out && (rc = ensure_host_staging(p, 1, one * (size_t)chunk, depth))) return rc;
-  cudaEventRecord(p->ev_start, p->stream);
-  cudaStreamWaitEvent(p->cin, p->ev_start, 0);
-  cudaStreamWaitEvent(p->cout, p->ev_start, 0);
   const long long nc = (count + chunk - 1) / chunk;
+  // small blocks of columns: the events between the streams cost more (3 of 37 us) than the streams give
+  const bool single = columns && nc == 1 && one * (size_t)count <= (1 << 20);
+  const cudaStream_t cin = single ? p->stream : p->cin, cout = single ? p->stream : p->cout;
+  if (!single)
+  {
+    cudaEventRecord(p->ev_start, p->stream);
+    cudaStreamWaitEvent(cin, p->ev_start, 0);
+    cudaStreamWaitEvent(cout, p->ev_start, 0);
+  }
   const int b0 = p->stage_next % depth;
   p->stage_next = (int)((b0 + nc) % depth);
   const int lag = depth - 1;  // chunks between a chunk's copy in and its copy out on the host
@@ -1034,23 +1040,29 @@ int exec_host_staged(fcb_plan p, const float2 *in, long long in_rs, float2 *out,
       src_pitch = k.rb;
     }
     float2 *buf = p->stage[b];
-    cudaStreamWaitEvent(p->cin, p->ev_out[b], 0);
-    cudaError_t e = copy(buf, k.rb, src, src_pitch, k, cudaMemcpyHostToDevice, p->cin);
+    cudaStreamWaitEvent(cin, p->ev_out[b], 0);
+    cudaError_t e = copy(buf, k.rb, src, src_pitch, k, cudaMemcpyHostToDevice, cin);
     if (e != cudaSuccess) return host_done(p, cuda_error(e, "host->device copy"), "fcb_exec (host)");
-    cudaEventRecord(p->ev_in[b], p->cin);
-    if (stage_in) cudaEventRecord(p->ev_h[0][b], p->cin);
-    cudaStreamWaitEvent(p->stream, p->ev_in[b], 0);
+    if (stage_in) cudaEventRecord(p->ev_h[0][b], cin);
+    if (!single)
+    {
+      cudaEventRecord(p->ev_in[b], cin);
+      cudaStreamWaitEvent(p->stream, p->ev_in[b], 0);
+    }
     rc = columns ? mixed_transform(p->mx, true, buf, k.k, buf, k.k, k.k, p->mode == kInv, p->scale, p->stream)
                  : exec_device(p, buf, p->n, buf, p->n, k.k, c * chunk, p->stream, 0);
     if (rc) return host_done(p, rc, "fcb_exec (host)");
-    cudaEventRecord(p->ev_k[b], p->stream);
-    cudaStreamWaitEvent(p->cout, p->ev_k[b], 0);
+    if (!single)
+    {
+      cudaEventRecord(p->ev_k[b], p->stream);
+      cudaStreamWaitEvent(cout, p->ev_k[b], 0);
+    }
     // the output's pinned buffer was drained on the host depth chunks ago
-    e = stage_out ? copy(pinned().buf[1][b], k.rb, buf, k.rb, k, cudaMemcpyDeviceToHost, p->cout)
-                  : copy(out + at(c, out_rs), sizeof(float2) * (size_t)out_rs, buf, k.rb, k, cudaMemcpyDeviceToHost, p->cout);
+    e = stage_out ? copy(pinned().buf[1][b], k.rb, buf, k.rb, k, cudaMemcpyDeviceToHost, cout)
+                  : copy(out + at(c, out_rs), sizeof(float2) * (size_t)out_rs, buf, k.rb, k, cudaMemcpyDeviceToHost, cout);
     if (e != cudaSuccess) return host_done(p, cuda_error(e, "device->host copy"), "fcb_exec (host)");
-    cudaEventRecord(p->ev_out[b], p->cout);
-    if (stage_out) cudaEventRecord(p->ev_h[1][b], p->cout);
+    cudaEventRecord(p->ev_out[b], cout);
+    if (stage_out) cudaEventRecord(p->ev_h[1][b], cout);
     if (stage_out && c >= lag)
     {
       rc = drain(c - lag);
@@ -1067,15 +1079,15 @@ int exec_host_staged(fcb_plan p, const float2 *in, long long in_rs, float2 *out,
 }
 
 // Columns on host pointers.  A side is staged where it is pageable, and where the copy
-// engine would move many short rows, about 36 ns each (pinned strided arrays, 20 columns of
+// engine would move many short rows, about 40 ns each (pinned strided arrays, 20 columns of
 // 2048 / 8000 / 14000: 233 / 766 / 1378 us moved as they are, 117 / 190 / 452 staged; but 20 of
-// 128 59 / 97, one of 8000 68 / 99, 100 of 8000 1028 / 834 with rows of 800 bytes).  Pageable
+// 128 59 / 97, 4 of 2048 112 / 103, one of 8000 68 / 99, 50 of 2048 242 / 235).  Pageable
 // arrays, 20 columns of 2048 / 14000: 116 / 478 us, 1144 of 756 573 us (with whole-array copies
 // one after the other 369 / 1622 / 1259, by transposing on the host 190 / 1108 / 3136).
 int exec_cols_host(fcb_plan p, const float2 *in, long long in_rs, float2 *out, long long out_rs, long long cols)
 {
   const long long n = p->n, chunk = std::min(cols, std::max<long long>(1, stage_bytes() / (8 * n)));
-  const bool short_rows = n >= 1000 && chunk > 1 && 8 * chunk < 512;
+  const bool short_rows = n >= 2000 && chunk >= 4 && chunk <= 32;
   auto staged = [&](const float2 *x, long long rs) {
     return (short_rows && rs != chunk) || host_pageable(x, sizeof(float2) * (size_t)((n - 1) * rs + cols));
   };

@@ -34,7 +34,7 @@ def test_threads_share_a_column_plan():
 
 
 @pytest.mark.parametrize("pinned", [False, True])
-@pytest.mark.parametrize("n,cols", [(2, 1), (16, 5), (999, 20), (1000, 20), (1000, 63), (1000, 64), (2048, 1), (14336, 9),
+@pytest.mark.parametrize("n,cols", [(2, 1), (16, 5), (1960, 20), (2000, 3), (2000, 4), (2000, 32), (2000, 33), (2048, 1), (14336, 9),
                                     (756, 2774), (756, 2775), (756, 9000), (14000, 400)])
 def test_blocks_and_strides_equal_the_device(n, cols, pinned):
     # one block, several (16 MB each) and their edges; packed, strided and in place
